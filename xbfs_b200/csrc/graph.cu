@@ -65,7 +65,10 @@ xbfs_status PinnedBuf::ensure(size_t n) {
   return XBFS_OK;
 }
 
+Graph::Graph() { ms_graph_created(); }
+
 Graph::~Graph() {
+  ms_graph_freed();
   DeviceGuard dg(device);
   if (ss.ev0) cudaEventDestroy(ss.ev0);
   if (ss.ev1) cudaEventDestroy(ss.ev1);

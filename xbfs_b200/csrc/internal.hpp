@@ -92,8 +92,16 @@ struct Graph {
   DevBuf head;                   // int4[V]: first three neighbours (-1 past the degree), degree
   cudaStream_t stream = nullptr;
   SsWorkspace ss;
+  Graph();
+  Graph(const Graph&) = delete;
+  Graph& operator=(const Graph&) = delete;
   ~Graph();
 };
+
+// msbfs.cu: graph handles alive; the last one to go frees the idle workspaces
+// of batched traversals
+void ms_graph_created();
+void ms_graph_freed();
 
 // RAII device guard
 struct DeviceGuard {
