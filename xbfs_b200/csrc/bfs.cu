@@ -153,6 +153,29 @@ constexpr long long kSpecEdges = 1 << 16;  // frontiers with at most this many e
 
 constexpr unsigned long long kCountMask = (1ull << 31) - 1;
 
+struct PolicyState {
+  // reference heuristic state (bfs_adaptiveFQ_wb_async.cuh:946-1078)
+  long long count_prev;
+  int is_change;
+  long long td_adaptive;
+  long long hub_before;
+  long long hub_after;
+  int tag_prev;  // 0: scan-free / last-phase TD, 1: second-phase TD, -1: BU
+  // Beamer
+  int bu_dir;
+  // features
+  long long n_prev;
+  int prev_strategy;
+};
+
+// Loop state handed back to every CTA at the end of a run of small levels.
+struct FewState {
+  long long L, vis_n, vis_m;
+  PolicyState ps;
+  float mlp_raw[8], mlp_margin;  // the learned switch's last evaluation
+  int mlp_dec;
+};
+
 struct FDesc {
   unsigned long long bin[3];  // packed: (edges << 31) | count
   unsigned long long n;       // vertices in the frontier (degree-0 included)
@@ -169,6 +192,17 @@ struct LevelRecDev {
   unsigned long long t0, t1;
 };
 
+// Small levels run by a few CTAs (small_levels).
+// 32 CTAs: their counts are one read per lane of a warp, and an exchange takes
+// 0.6 us (64: 0.74, 148: 2.3); 16 CTAs take 4.8 us a level of the 4096 x 4096
+// grid against 3.2, 24 take 3.8.
+constexpr int kFew = 32;                  // CTAs that share a run of small levels
+constexpr int kFewEdges = 2048;           // frontier edges a CTA can hold
+constexpr int kFewShare = 1536;           // and may start with (mean over the CTAs)
+constexpr int kSoloIn = 512, kSoloOut = 768;  // one CTA alone: enters with at most, leaves above
+constexpr int kFewOut = 192;              // several CTAs: leave (for one alone) below
+constexpr int kFewAfter = 6;              // levels in a row that would have fitted before a run starts
+
 struct Ctl {
   GridBarrier bar;
   int depth;
@@ -178,6 +212,14 @@ struct Ctl {
   unsigned long long heavy[2];  // packed counter of the heavy list, by level parity
   int strat_count[4];
   FDesc fd[4];
+  // runs of small levels: what each CTA found at a level (level + 1 in the
+  // upper word), by level parity; the frontier handed back, by run; CTAs that
+  // wait for a run's end, since launch; the running level
+  unsigned long long few[2][kFew];
+  FDesc back[3];
+  unsigned int waiting;
+  unsigned long long progress;
+  FewState state;
 };
 
 struct QBin {
@@ -231,20 +273,15 @@ __device__ __forceinline__ int bin_of(long long d, int small_max, int medium_max
 // ---------------------------------------------------------------------------
 // Strategy policy (computed identically by thread 0 of every CTA).
 // ---------------------------------------------------------------------------
-struct PolicyState {
-  // reference heuristic state (bfs_adaptiveFQ_wb_async.cuh:946-1078)
-  long long count_prev;
-  int is_change;
-  long long td_adaptive;
-  long long hub_before;
-  long long hub_after;
-  int tag_prev;  // 0: scan-free / last-phase TD, 1: second-phase TD, -1: BU
-  // Beamer
-  int bu_dir;
-  // features
-  long long n_prev;
-  int prev_strategy;
+// Runs of small levels, learned switch: what the statistics of a level may be
+// for the network to be sure to pick XBFS_TD_QUEUE (see few_box).
+struct FewSure {
+  unsigned n_lo, n_hi, m_lo, m_hi;  // vertices, degree sum
+  unsigned vn_hi, vm_hi, level_hi;  // visited sums with this level's, level
+  float d_lo, d_hi;                 // degree sum over vertices
+  float g_lo, g_hi;                 // vertices + 1 over the level before's
 };
+constexpr int kFewRing = 16;
 
 // Per-CTA loop state owned by thread 0 (in shared memory).
 struct LoopState {
@@ -291,7 +328,26 @@ struct __align__(16) Smem {
   int mlp_cache_dec;            // and its decision (-1: none yet)
   float mlp_cache_margin;       // and that decision's margin
   float mlp_q[8];               // sensitivity bound per feature over the feature's scale
+  __align__(16) float mlp_act[32];  // activations of the network being evaluated
   LoopState ls;
+  int few;                      // CTAs that run the next levels alone (0: a level of the whole grid)
+  int few_exit;                 // the run ends before the next level
+  unsigned few_edges[2], few_n[2];  // edges and vertices found, by parity of the level that finds them
+  unsigned few_spill[2];        // some of them went to the global queue
+  unsigned long long few_m[2];  // degree sum of those with too many edges for the run
+  // statistics posted for the last warp, a ring by level: n_f, m_f, the visited
+  // sums, the vertices of the level before; the level posted last (~0: the run
+  // is over) and the one it has dealt with
+  unsigned few_rec[kFewRing][5];
+  volatile unsigned few_seq, few_seen;
+  FewSure few_sure[2];          // what that warp is sure of, by the parity of few_made
+  volatile unsigned few_made;
+  __align__(16) float few_act[32];  // its evaluation's activations and statistics
+  float few_raw[8];
+  float few_margin;
+  int few_dec;
+  int fitted;                   // levels in a row that would have fitted a run
+  unsigned waiting;             // thread 0: CTAs that have waited for runs' ends so far
   float mlp_w[1472];            // the learned switch's weights and bound (XBFS_POLICY_MLP); must stay last
 };
 
@@ -400,16 +456,14 @@ __device__ void mlp_stage(const float* __restrict__ w, float* sw) {
 // levels (a grid's ring of a few thousand vertices growing by a few per
 // level) then cost a few scalar operations, and decisions are those of
 // evaluating the network at every level.
-__device__ int mlp_decide(const float* sw, const float* raw, int lane, float* cache_raw, int* cache_dec,
-                          float* cache_margin) {
+// In two parts, so that a run of small levels can spread an evaluation over
+// two levels: mlp_first leaves the first layer's activations in act (shared
+// memory, read back four per broadcast), mlp_second does the rest.
+__device__ __forceinline__ void mlp_first(const float* sw, const float* raw, float* act, int lane) {
   const float* mean = sw;
   const float* sd = sw + 8;
   const float* W1T = sw + 16;
   const float* B1 = W1T + 256;
-  const float* W2T = B1 + 32;
-  const float* B2 = W2T + 1024;
-  const float* W3 = B2 + 32;
-  const float* B3 = W3 + 96;
   float f = 0.f;
   if (lane < 8) {
     const float r = raw[lane];
@@ -418,14 +472,40 @@ __device__ int mlp_decide(const float* sw, const float* raw, int lane, float* ca
     else f = log1pf(r > 0.f ? r : 0.f);
     f = (f - mean[lane]) / sd[lane];
   }
+  const float4* act4 = reinterpret_cast<const float4*>(act);
+  if (lane < 8) act[lane] = f;
+  __syncwarp();
   float a = B1[lane];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) a = fmaf(W1T[i * 32 + lane], __shfl_sync(0xffffffffu, f, i), a);
-  a = fmaxf(a, 0.f);
+  for (int i = 0; i < 8; i += 4) {
+    const float4 t = act4[i / 4];
+    a = fmaf(W1T[i * 32 + lane], t.x, a);
+    a = fmaf(W1T[(i + 1) * 32 + lane], t.y, a);
+    a = fmaf(W1T[(i + 2) * 32 + lane], t.z, a);
+    a = fmaf(W1T[(i + 3) * 32 + lane], t.w, a);
+  }
+  __syncwarp();
+  act[lane] = fmaxf(a, 0.f);
+  __syncwarp();
+}
+
+__device__ __forceinline__ int mlp_second(const float* sw, const float* raw, const float* act, int lane,
+                                          float* cache_raw, int* cache_dec, float* cache_margin) {
+  const float* W2T = sw + 16 + 256 + 32;
+  const float* B2 = W2T + 1024;
+  const float* W3 = B2 + 32;
+  const float* B3 = W3 + 96;
+  const float4* act4 = reinterpret_cast<const float4*>(act);
   // four independent accumulators shorten the dependent FMA chain of layer 2
   float bq[4] = {B2[lane], 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int i = 0; i < 32; ++i) bq[i & 3] = fmaf(W2T[i * 32 + lane], __shfl_sync(0xffffffffu, a, i), bq[i & 3]);
+  for (int i = 0; i < 32; i += 4) {
+    const float4 t = act4[i / 4];
+    bq[0] = fmaf(W2T[i * 32 + lane], t.x, bq[0]);
+    bq[1] = fmaf(W2T[(i + 1) * 32 + lane], t.y, bq[1]);
+    bq[2] = fmaf(W2T[(i + 2) * 32 + lane], t.z, bq[2]);
+    bq[3] = fmaf(W2T[(i + 3) * 32 + lane], t.w, bq[3]);
+  }
   const float b = fmaxf((bq[0] + bq[1]) + (bq[2] + bq[3]), 0.f);
   float o[3];
 #pragma unroll
@@ -447,6 +527,11 @@ __device__ int mlp_decide(const float* sw, const float* raw, int lane, float* ca
   return best;
 }
 
+__device__ int mlp_decide(const float* sw, const float* raw, float* act, int lane, float* cache_raw, int* cache_dec,
+                          float* cache_margin) {
+  mlp_first(sw, raw, act, lane);
+  return mlp_second(sw, raw, act, lane, cache_raw, cache_dec, cache_margin);
+}
 
 // Upper bound (with a rounding allowance) of sum_i P[i] |x_i - x_last_i| from
 // the raw statistics a (now) and b (last evaluation), q[i] = P[i] / scale_i:
@@ -2182,17 +2267,613 @@ __device__ void init_traversal(const Params& p) {
   }
 }
 
+// Strategy of level L by the launch's policy, the learned switch's excepted.
+__device__ __forceinline__ int decide(const Params& p, PolicyState& ps, long long L, long long n_f, long long m_f,
+                                      long long m_u) {
+  switch (p.policy) {
+    case XBFS_POLICY_FORCED: {
+      const long long i = L < p.n_forced ? L : p.n_forced - 1;
+      const int s = (i >= 0) ? (int)p.forced[i] : XBFS_TD_QUEUE;
+      return s < 0 || s > 2 ? XBFS_TD_QUEUE : s;
+    }
+    case XBFS_POLICY_BEAMER:
+      return decide_beamer(ps, n_f, m_f, m_u, p.V, p.beamer_alpha, p.beamer_beta);
+    default:
+      return decide_reference(ps, L, m_f, p.E, p.alpha);
+  }
+}
+
+// The learned switch (thread 0): its last decision where that is certified,
+// else -2 with the statistics in sm.mlp_raw for warp 0 to evaluate the network.
+__device__ __forceinline__ int decide_learned(Smem& sm, long long L, long long n_f, long long m_f, long long n_u,
+                                              long long m_u) {
+  const PolicyState& ps = sm.ls.ps;
+  const float raw[8] = {(float)n_f, (float)m_f, (float)n_u, (float)m_u, (float)L,
+                        (float)ps.prev_strategy, (float)ps.n_prev, (float)m_f / (float)n_f};
+  if (sm.mlp_cache_dec >= 0 && mlp_reuse_bound(raw, sm.mlp_cache_raw, sm.mlp_q) < sm.mlp_cache_margin)
+    return sm.mlp_cache_dec;  // certified: the network would choose the same
+#pragma unroll
+  for (int k = 0; k < 8; ++k) sm.mlp_raw[k] = raw[k];
+  return -2;
+}
+
+// ---------------------------------------------------------------------------
+// Runs of small top-down levels.
+// ---------------------------------------------------------------------------
+// A level of a few thousand edges does not need the grid: its cost is the
+// chain from one frontier to the next (descriptor, queue entry, CSR, claim,
+// queue slot, grid barrier): 6.6 us on an 8192 x 16 grid graph, 8.3 on a
+// 4096 x 4096 one (3,000 vertices a level); in a run 2.2 and 3.5. Here kFew CTAs (one alone for up to
+// kSoloOut edges) run such levels while the others wait. Every CTA keeps the
+// edges of the frontier vertices it found itself in shared memory, one CSR
+// position per edge. A level is then
+//   claims      one atomic on the visited bitmap per edge; the winners' edges
+//               go to the next level's shared-memory list
+//   barrier A
+//   warp 0      counts: each CTA writes one word and reads all of them (no
+//               atomics), then the next strategy
+//   the others  read the next level's targets and their CSR offsets meanwhile
+//   barrier B
+// so that the CSR reads are off the critical path; the last warp keeps the
+// records beside it (few_aside). The run ends when the policy
+// picks another strategy, the frontier outgrows it (or shrinks to what one CTA
+// does faster), its edges gather in few CTAs, or a vertex of more than
+// small_max edges or more edges than fit was found; what is left in shared
+// memory then becomes the binned queue again. Entering and leaving costs about
+// what a level of the whole grid does, so a run starts after kFewAfter levels
+// that would have fitted (R-MAT and Erdos-Renyi graphs have up to five).
+struct FewSmem {
+  unsigned pos[2][kFewEdges];  // CSR position of every frontier edge, by level parity
+  int u[2][kFewEdges];         // the frontier vertex it belongs to
+};
+static_assert(sizeof(FewSmem) <= offsetof(Smem, stl_id), "runs of small levels live in the window and staging areas");
+constexpr int kFewThreads = kBlock - 64;  // threads that take edges (warp 0 exchanges and decides, the last keeps records)
+constexpr int kFewK = 2;                  // edges per thread read ahead (1: 4.4 us a level of the 4096 x 4096 grid, not 3.4)
+
+// Puts vertex v's d edges (CSR offset b0) at edge slot `at` of the frontier.
+__device__ __forceinline__ void few_put(FewSmem& fs, int par, unsigned at, int v, unsigned d, unsigned b0) {
+  for (unsigned j = 0; j < d; ++j) {
+    fs.pos[par][at + j] = b0 + j;
+    fs.u[par][at + j] = v;
+  }
+}
+
+// kFewK edges of a thread: target and its CSR offsets (as read: nothing waits
+// for them before the claims).
+struct FewEdges {
+  int v[kFewK];
+  long long b0[kFewK], b1[kFewK];
+};
+
+// Reads the targets of frontier edges e, e + kFewThreads, ... < m.
+__device__ __forceinline__ void few_load(const Params& p, const FewSmem& fs, int par, unsigned e, unsigned m,
+                                         FewEdges& x) {
+#pragma unroll
+  for (int k = 0; k < kFewK; ++k)
+    x.v[k] = e + k * kFewThreads < m ? __ldg(p.csr + fs.pos[par][e + k * kFewThreads]) : -1;
+#pragma unroll
+  for (int k = 0; k < kFewK; ++k) {
+    x.b0[k] = 0;
+    x.b1[k] = 0;
+    if (x.v[k] >= 0) {
+      x.b0[k] = ld_nc_i64(p.beg + x.v[k]);
+      x.b1[k] = ld_nc_i64(p.beg + x.v[k] + 1);
+    }
+  }
+}
+
+// Claims the targets x (edges e, e + kFewThreads, ... of level L's frontier)
+// for level L+1. Winners without edges only count. Full warps.
+template <bool PAR>
+__device__ __forceinline__ void few_claim(const Params& p, Smem& sm, FewSmem& fs, FDesc* back, int L, unsigned e,
+                                          const FewEdges& x) {
+  const int par = L & 1, lane = threadIdx.x & 31;
+  uint32_t old[kFewK];
+#pragma unroll
+  for (int k = 0; k < kFewK; ++k)
+    old[k] = x.v[k] >= 0 ? atomicOr(p.vis + (x.v[k] >> 5), 1u << (x.v[k] & 31)) : ~0u;
+  unsigned won = 0, d[kFewK], kd[kFewK], sum = 0;
+#pragma unroll
+  for (int k = 0; k < kFewK; ++k) {
+    const bool win = x.v[k] >= 0 && !((old[k] >> (x.v[k] & 31)) & 1u);
+    d[k] = (unsigned)(x.b1[k] - x.b0[k]);
+    kd[k] = win && d[k] <= (unsigned)p.small_max ? d[k] : 0u;
+    sum += kd[k];
+    if (win) {
+      won |= 1u << k;
+      p.levels[x.v[k]] = L + 1;
+      if (PAR) p.parents[x.v[k]] = fs.u[par][e + k * kFewThreads];
+    }
+  }
+  if (!__ballot_sync(0xffffffffu, won)) return;
+  const unsigned n = __reduce_add_sync(0xffffffffu, __popc(won));
+  const unsigned inc = warp_inclusive_scan(sum);
+  unsigned at = 0;
+  if (lane == 31) {
+    if (inc) at = atomicAdd(&sm.few_edges[par], inc);
+    atomicAdd(&sm.few_n[par], n);
+  }
+  at = __shfl_sync(0xffffffffu, at, 31) + inc - sum;
+#pragma unroll
+  for (int k = 0; k < kFewK; ++k) {
+    if (!((won >> k) & 1u) || d[k] == 0) continue;
+    if (kd[k] && at + kd[k] <= kFewEdges) {
+      few_put(fs, par ^ 1, at, x.v[k], kd[k], (unsigned)x.b0[k]);
+    } else {
+      // too many edges, in all or of this vertex: the global queue of the
+      // next level, which the whole grid then runs
+      const int bin = bin_of(d[k], p.small_max, p.medium_max);
+      direct_enqueue(p.q[par ^ 1][bin], &back->bin[bin], x.v[k], d[k], x.b0[k]);
+      if (kd[k]) {  // the slots it leaves unused are no vertex's (and read ahead all the same)
+        for (unsigned j = at; j < min(at + kd[k], (unsigned)kFewEdges); ++j) {
+          fs.pos[par ^ 1][j] = 0;
+          fs.u[par ^ 1][j] = -1;
+        }
+      } else {
+        atomicAdd(&sm.few_m[par], (unsigned long long)d[k]);
+      }
+      sm.few_spill[par] = 1u;
+    }
+    at += kd[k];
+  }
+}
+
+// Statistics of a run's level: vertices, degree sum, the visited sums (this
+// level included), level, vertices of the level before.
+struct FewStat {
+  unsigned n, m, vn, vm, level, prev;
+};
+
+// Learned switch: the box around an evaluation of the network at level t, a
+// range of each statistic the features come from (n_f, m_f, n_u, m_u, level,
+// growth (n_f + 1) / (n_prev + 1), mean degree) within which, all together, the
+// network is sure to pick XBFS_TD_QUEUE: the margin of its decision is spread
+// over the features (see mlp_reuse_bound), of which the first five may each
+// move by the relative amount r, and the growth and the mean degree, which
+// hardly change in a run, by r / 4. Called by a full warp; `sure` in, the new
+// box (of nothing when the margin is used up) out.
+__device__ __noinline__ FewSure few_box(const Params& p, Smem& sm, const FewStat& t) {
+  const int lane = threadIdx.x & 31;
+  const float n = (float)t.n, m = (float)t.m, n_u = (float)max(p.n_ni - (long long)t.vn, 0ll),
+              m_u = (float)max(p.E - (long long)t.vm, 0ll), level = (float)t.level, g = (n + 1.f) / ((float)t.prev + 1.f),
+              d = m / n;
+  if (lane == 0) {
+    float* raw = sm.few_raw;
+    raw[0] = n;
+    raw[1] = m;
+    raw[2] = n_u;
+    raw[3] = m_u;
+    raw[4] = level;
+    raw[5] = (float)XBFS_TD_QUEUE;
+    raw[6] = (float)t.prev;
+    raw[7] = d;
+  }
+  __syncwarp();
+  mlp_first(sm.mlp_w, sm.few_raw, sm.few_act, lane);
+  mlp_second(sm.mlp_w, sm.few_raw, sm.few_act, lane, sm.few_raw, &sm.few_dec, &sm.few_margin);
+  const float* q = sm.mlp_q;
+  const float w = q[0] + q[1] + q[2] + q[3] + q[4] + 0.25f * (q[6] + q[7]);
+  const float margin = sm.few_dec == XBFS_TD_QUEUE ? sm.few_margin : 0.f;
+  const float r = w > 0.f ? fminf(0.95f * (margin - 1e-5f) / (1.02f * w), 0.2f) : 0.f;
+  if (!(r > 1e-5f)) return FewSure{1u, 0u, 0u, 0u, 0u, 0u, 0u, 0.f, 0.f, 0.f, 0.f};
+  // within r of c: (u - c) / (1 + c) <= r upwards, (c - u) / (1 + u) <= r
+  // downwards; the growth's logarithm moves by at most |u - c| / min(u, c)
+  const float down = 1.f / (1.f + r), r4 = 0.25f * r, down4 = 1.f / (1.f + r4);
+  FewSure b;
+  b.n_lo = (unsigned)fmaxf(ceilf((n - r) * down), 0.f);
+  b.n_hi = (unsigned)(n + r * (1.f + n));
+  b.m_lo = (unsigned)fmaxf(ceilf((m - r) * down), 0.f);
+  b.m_hi = (unsigned)(m + r * (1.f + m));
+  // n_u and m_u fall by what gets visited
+  b.vn_hi = t.vn + (unsigned)fmaxf(n_u - (n_u - r) * down, 0.f);
+  b.vm_hi = t.vm + (unsigned)fmaxf(m_u - (m_u - r) * down, 0.f);
+  b.level_hi = (unsigned)(level + r * (1.f + level));
+  b.d_lo = (d - r4) * down4;
+  b.d_hi = d + r4 * (1.f + d);
+  b.g_lo = g * down4;
+  b.g_hi = g + r4 * g;
+  return b;
+}
+
+// Whether a level of these statistics lies in the box.
+__device__ __forceinline__ bool few_inside(const FewSure& b, unsigned n, unsigned m, unsigned vn, unsigned vm,
+                                           unsigned level, unsigned prev) {
+  const float nf = (float)n, mf = (float)m, pf = (float)prev + 1.f;
+  return n >= b.n_lo && n <= b.n_hi && m >= b.m_lo && m <= b.m_hi && vn <= b.vn_hi && vm <= b.vm_hi &&
+         level <= b.level_hi && mf >= b.d_lo * nf && mf <= b.d_hi * nf && nf + 1.f >= b.g_lo * pf &&
+         nf + 1.f <= b.g_hi * pf;
+}
+
+// The last warp of a run's CTA, beside the levels: block 0's writes the
+// levels' records; with the learned switch it keeps a box (few_box) drawn around
+// a recent level, so that warp 0 seldom has to evaluate the network between
+// two levels. It follows warp 0 through few_seq and takes no part in the
+// levels' barriers.
+template <bool MLP>
+__device__ __noinline__ void few_aside(const Params& p, Smem& sm, unsigned L0) {
+  const int lane = threadIdx.x & 31;
+  const bool records = blockIdx.x == 0;
+  FewSure b{1u, 0u, 0u, 0u, 0u, 0u, 0u, 0.f, 0.f, 0.f, 0.f};
+  FewSure h = b;  // the part of it after which a new one is drawn
+  unsigned made = 0;
+  for (unsigned next = L0 + 1;; ++next) {
+    unsigned seq;
+    for (;;) {
+      seq = sm.few_seq;
+      if (seq == ~0u || (int)(seq - next) >= 0) break;
+      __nanosleep(40);
+    }
+    if (seq == ~0u) return;
+    __threadfence_block();
+    const unsigned* rec = sm.few_rec[next % kFewRing];
+    FewStat t{rec[0], rec[1], rec[2], rec[3], next, rec[4]};
+    if (records && lane == 0) {
+      st_relaxed_u64(&p.ctl->progress, (unsigned long long)next);
+      if ((long long)next < p.hist_cap) {
+        LevelRecDev& r = p.hist[next];
+        r.n_f = t.n;
+        r.m_f = t.m;
+        r.n_u = max(p.n_ni - (long long)t.vn, 0ll);
+        r.m_u = max(p.E - (long long)t.vm, 0ll);
+        r.strategy = XBFS_TD_QUEUE;
+        r.t0 = globaltimer_ns();
+        r.t1 = 0;
+        p.hist[next - 1].t1 = r.t0;
+      }
+    }
+    if (MLP && seq == next && !few_inside(h, t.n, t.m, t.vn, t.vm, t.level, t.prev)) {
+      b = few_box(p, sm, t);
+      h = b;
+      if (b.n_hi >= b.n_lo) {
+        h.n_lo = t.n - (t.n - min(b.n_lo, t.n)) / 2;
+        h.n_hi = t.n + (b.n_hi - t.n) / 2;
+        h.m_lo = t.m - (t.m - min(b.m_lo, t.m)) / 2;
+        h.m_hi = t.m + (b.m_hi - t.m) / 2;
+        h.vn_hi = t.vn + (b.vn_hi - t.vn) / 2;
+        h.vm_hi = t.vm + (b.vm_hi - t.vm) / 2;
+        h.level_hi = t.level + (b.level_hi - t.level) / 2;
+      }
+      __syncwarp();
+      if (lane == 0) {
+        // warp 0 reads the other buffer until few_made moves on
+        sm.few_sure[(made + 1) & 1] = b;
+        __threadfence_block();
+        sm.few_made = made + 1;
+      }
+      ++made;
+    }
+    __syncwarp();
+    if (lane == 0) sm.few_seen = next;
+  }
+}
+
+// Learned switch: decision for a level outside the box (full warp).
+// t: the level before the one to decide.
+__device__ __noinline__ int few_decide_learned(const Params& p, Smem& sm, const FewStat& t, unsigned n, unsigned m) {
+  const int lane = threadIdx.x & 31;
+  int s = XBFS_TD_QUEUE;
+  if (lane == 0) {
+    sm.ls.ps.n_prev = t.n;
+    s = decide_learned(sm, (long long)t.level + 1, n, m, max(p.n_ni - (long long)t.vn - n, 0ll),
+                       max(p.E - (long long)t.vm - m, 0ll));
+  }
+  s = __shfl_sync(0xffffffffu, s, 0);
+  if (s == -2) {
+    s = mlp_decide(sm.mlp_w, sm.mlp_raw, sm.mlp_act, lane, sm.mlp_cache_raw, &sm.mlp_cache_dec, &sm.mlp_cache_margin);
+    s = __shfl_sync(0xffffffffu, s, 0);
+  }
+  __syncwarp();
+  return s;
+}
+
+// Counts of one level across the run's CTAs (full warp): each writes one word
+// tagged with the level, reads all of them and sums: vertices (12 bits, a level
+// finds at most kFewEdges per CTA), edges (12 bits), spill; mx is the largest
+// edge count. False when the others' words do not come within the time limit.
+// The words need no release or acquire: what the next level reads of other
+// CTAs' work is the visited bitmap, only by atomics, and every claim of this
+// level has returned its old value (all warps have passed the block barrier on
+// it) before the word is written; the rest is published by the grid barrier
+// that ends the run. A fence here costs 0.4 us of a level's 3.6.
+__device__ __forceinline__ bool few_exchange(const Params& p, int N, unsigned tag, unsigned& n, unsigned& m,
+                                             unsigned& mx, unsigned& spill) {
+  unsigned long long* f = p.ctl->few[tag & 1];
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) st_relaxed_u64(f + blockIdx.x, ((unsigned long long)tag << 32) | (spill << 24) | (m << 12) | n);
+  unsigned long long w = 0, t0 = 0;
+  uint32_t spins = 0;
+  for (;;) {
+    bool here = true;
+    if (lane < N) {
+      w = ld_relaxed_u64(f + lane);
+      here = (unsigned)(w >> 32) == tag;
+    }
+    if (__all_sync(0xffffffffu, here)) break;
+    if ((++spins & 1023u) == 0) {
+      if (t0 == 0) t0 = globaltimer_ns();
+      const bool late = globaltimer_ns() - t0 > p.timeout_ns;
+      if (late && lane == 0) atomicCAS(&p.ctl->bar.err, 0, (int)XBFS_ERR_DEVICE_TIMEOUT);
+      if (__any_sync(0xffffffffu, late || ld_acquire_i32(&p.ctl->bar.err) != 0)) return false;
+    }
+  }
+  const unsigned y = lane < N ? (unsigned)w : 0u;
+  n = __reduce_add_sync(0xffffffffu, y & 0xfffu);
+  m = __reduce_add_sync(0xffffffffu, (y >> 12) & 0xfffu);
+  mx = __reduce_max_sync(0xffffffffu, (y >> 12) & 0xfffu);
+  spill = __reduce_or_sync(0xffffffffu, y >> 24);
+  return true;
+}
+
+// Runs levels from L on with sm.few CTAs (block 0 first), the others waiting;
+// `run` counts the launch's runs before this one. Leaves the frontier of the
+// returned level in the binned queue and ctl->back[run % 3], every frontier
+// bitmap empty, the same loop state in every CTA and the level in red4[0], and
+// passes one grid barrier. False: the launch has to end (time limit).
+template <bool PAR, bool LEARNED>
+__device__ __noinline__ bool small_levels(const Params& p, Smem& sm, long long L, uint32_t epoch, unsigned dirty,
+                                          unsigned run) {
+  Ctl* ctl = p.ctl;
+  LoopState& ls = sm.ls;
+  FewSmem& fs = *reinterpret_cast<FewSmem*>(&sm);
+  const int N = sm.few;
+  const uint32_t nb = gridDim.x;
+  const int lane = threadIdx.x & 31;
+  FDesc* back = &ctl->back[run % 3];
+  for (int i = 0; i < 4; ++i)
+    if (dirty & (1u << i)) clear_bitmap(p.fb[i], p.nwords);
+  if ((int)blockIdx.x >= N) {
+    __syncthreads();
+    if (threadIdx.x == 0) red_add_release_u32(&ctl->waiting, 1u);
+    if (!grid_sync(&ctl->bar, nb, epoch, p.timeout_ns, &ctl->progress)) return false;
+  } else {
+    // this CTA's part of the small bin: the entries whose first edge lies in
+    // its share of the edges
+    const QBin& in = p.q[L & 1][0];
+    const unsigned cnt = (unsigned)(sm.bins[0] & kCountMask);
+    const unsigned M = (unsigned)(sm.bins[0] >> 31);
+    if (threadIdx.x < 64) {
+      const int c = (int)blockIdx.x + (threadIdx.x >> 5);
+      const unsigned key = (unsigned)((unsigned long long)M * c / N);
+      int s = (int)cnt;
+      if (c < N) {
+        s = find_owner(in.eb, cnt, key);
+        if (in.eb[s] != key) ++s;
+      }
+      if (lane == 0) sm.red4[threadIdx.x >> 5] = s;
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 8)  // the descriptor of the next run (last read before the previous one)
+      reinterpret_cast<unsigned long long*>(&ctl->back[(run + 1) % 3])[threadIdx.x] = 0ull;
+    if (threadIdx.x == 0) ls.ps.prev_strategy = XBFS_TD_QUEUE;
+    if (threadIdx.x < 2) {
+      sm.few_edges[threadIdx.x] = sm.few_n[threadIdx.x] = sm.few_spill[threadIdx.x] = 0;
+      sm.few_m[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    const unsigned s0 = (unsigned)sm.red4[0], s1 = (unsigned)sm.red4[1];
+    const unsigned base = s0 < cnt ? in.eb[s0] : M;
+    unsigned m = (s1 < cnt ? in.eb[s1] : M) - base;
+    for (unsigned i = s0 + threadIdx.x; i < s1; i += kBlock) {
+      const unsigned e = in.eb[i], e1 = i + 1 < cnt ? in.eb[i + 1] : M;
+      few_put(fs, (int)(L & 1), e - base, in.ids[i], e1 - e, (unsigned)in.bg[i]);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      sm.few_seq = sm.few_seen = (unsigned)L;
+      sm.few_made = 0;
+      sm.few_sure[0] = FewSure{1u, 0u, 0u, 0u, 0u, 0u, 0u, 0.f, 0.f, 0.f, 0.f};
+    }
+    __syncthreads();
+    const unsigned L0 = (unsigned)L;
+    if (threadIdx.x >= kBlock - 32) {
+      few_aside<LEARNED>(p, sm, L0);
+    } else {
+      // barriers of the other warps only
+      auto level_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(kBlock - 32) : "memory"); };
+      const unsigned e0 = threadIdx.x - 32u;  // this thread's first edge (warps 1 and up)
+      FewEdges x;
+      if (threadIdx.x >= 32) few_load(p, fs, (int)(L & 1), e0, m, x);
+      // warp 0: the running level's statistics; the entry level's own decision
+      // was the level loop's
+      const unsigned max_l = (unsigned)(p.max_levels - 1);
+      FewStat st{(unsigned)ls.ps.n_prev, M, (unsigned)ls.vis_n, (unsigned)ls.vis_m, L0, 0u};
+      PolicyState ps = ls.ps;
+      FewSure sure{1u, 0u, 0u, 0u, 0u, 0u, 0u, 0.f, 0.f, 0.f, 0.f};
+      for (;;) {
+        const int par = (int)(L & 1);
+        if (LEARNED && threadIdx.x < 32) {
+          // the box as it is now, while the others claim
+          const unsigned made = sm.few_made;
+          sure = sm.few_sure[made & 1];
+          if (sm.few_made != made) sure.n_lo = ~0u;  // being drawn anew
+        }
+        if (threadIdx.x >= 32 && (e0 & ~31u) < m) {  // whole warps
+          for (unsigned e = e0;;) {
+            few_claim<PAR>(p, sm, fs, back, (int)L, e, x);
+            e += kFewK * kFewThreads;
+            if ((e & ~31u) >= m) break;
+            few_load(p, fs, par, e, m, x);
+          }
+        }
+        level_barrier();  // A
+        m = min(sm.few_edges[par], (unsigned)kFewEdges);
+        if (threadIdx.x < 32) {
+          unsigned n_s = sm.few_n[par], m_s = m, m_x = m, sp = sm.few_spill[par];
+          bool ok = true;
+          if (N > 1) ok = few_exchange(p, N, (unsigned)L + 1, n_s, m_s, m_x, sp);
+          // uneven: one CTA holds over twice its share and more than is read ahead
+          const bool uneven = N > 1 && m_x > (unsigned)(kFewK * kFewThreads) && m_x * N > 2 * m_s;
+          const bool size =
+              N > 1 ? (m_s > (unsigned)(N * kFewShare) || m_s < (unsigned)kFewOut) : m_s > (unsigned)kSoloOut;
+          int ex = !ok ? 2 : ((sp || uneven || size || n_s == 0 || (unsigned)L >= max_l) ? 1 : 0);
+          if (!ex) {
+            // the next level's decision, as the level loop would take it
+            PolicyState next = ps;
+            int s = XBFS_TD_QUEUE;
+            if (LEARNED) {
+              if (!few_inside(sure, n_s, m_s, st.vn + n_s, st.vm + m_s, st.level + 1, st.n))
+                s = few_decide_learned(p, sm, st, n_s, m_s);
+            } else {
+              s = decide(p, next, (long long)st.level + 1, n_s, m_s, max(p.E - (long long)st.vm - m_s, 0ll));
+            }
+            if (s == XBFS_BU && !p.allow_bu) s = XBFS_TD_QUEUE;
+            if (s == XBFS_TD_QUEUE)
+              ps = next;
+            else
+              ex = 1;  // the level loop decides it again
+          }
+          if (!ex) {
+            st.prev = st.n;
+            st.n = n_s;
+            st.m = m_s;
+            st.vn += n_s;
+            st.vm += m_s;
+            st.level += 1;
+            // for the last warp, which is never a ring behind
+            while ((int)(st.level - sm.few_seen) >= kFewRing) __nanosleep(20);
+            if (lane == 0) {
+              unsigned* rec = sm.few_rec[st.level % kFewRing];
+              rec[0] = n_s;
+              rec[1] = m_s;
+              rec[2] = st.vn;
+              rec[3] = st.vm;
+              rec[4] = st.prev;
+              __threadfence_block();
+              sm.few_seq = st.level;
+            }
+          }
+          if (lane == 0) sm.few_exit = ex;
+        } else {
+          if (threadIdx.x == 32) {
+            sm.few_edges[par ^ 1] = sm.few_n[par ^ 1] = sm.few_spill[par ^ 1] = 0;
+            sm.few_m[par ^ 1] = 0;
+          }
+          few_load(p, fs, par ^ 1, e0, m, x);
+        }
+        level_barrier();  // B
+        ++L;
+        if (sm.few_exit) break;
+      }
+      if (threadIdx.x == 0) {
+        // the loop state as the level loop would have left it
+        if (blockIdx.x == 0) {
+          ls.st_reached += st.vn - (unsigned)ls.vis_n;
+          ls.st_msum += st.vm - (unsigned)ls.vis_m;
+          ls.st_strat[XBFS_TD_QUEUE] += (int)((unsigned)L - L0);
+          if ((long long)L0 < p.hist_cap) p.hist[L0].strategy = XBFS_TD_QUEUE;
+        }
+        ls.vis_n = st.vn;
+        ls.vis_m = st.vm;
+        ls.ps = ps;
+        ls.ps.n_prev = st.n;
+        sm.red4[0] = L;
+        sm.few_rec[0][0] = m;
+        // the last warp may still have records to write
+        while ((int)(st.level - sm.few_seen) > 0) __nanosleep(20);
+        sm.few_seq = ~0u;
+      }
+    }
+    __syncthreads();
+    if (sm.few_exit == 2) return false;
+    L = sm.red4[0];
+    m = sm.few_rec[0][0];
+    const int par = (int)(L & 1);  // what level L-1 found, counted under par ^ 1
+    // ---- back to the whole grid: the edges' vertices into the small bin
+    for (unsigned f0 = 0; f0 < m; f0 += kBlock) {
+      const unsigned e = f0 + threadIdx.x;
+      bool have = false;
+      int v = 0;
+      long long b0 = 0, d = 0;
+      if (e < m) {
+        v = fs.u[par][e];
+        if (v >= 0) {
+          b0 = ld_nc_i64(p.beg + v);
+          have = fs.pos[par][e] == (unsigned)b0;  // v's first edge
+          if (have) d = ld_nc_i64(p.beg + v + 1) - b0;
+        }
+      }
+      const unsigned mask = __ballot_sync(0xffffffffu, have);
+      if (!mask) continue;
+      const long long inc = warp_inclusive_scan(d);
+      unsigned long long old = 0;
+      if (lane == 31)
+        old = atomicAdd(&back->bin[0], ((unsigned long long)inc << 31) | (unsigned long long)__popc(mask));
+      old = __shfl_sync(0xffffffffu, old, 31);
+      if (have) {
+        const unsigned slot = (unsigned)(old & kCountMask) + __popc(mask & ((1u << lane) - 1));
+        p.q[par][0].ids[slot] = v;
+        p.q[par][0].eb[slot] = (unsigned)((old >> 31) + (unsigned long long)(inc - d));
+        p.q[par][0].bg[slot] = b0;
+      }
+    }
+    if (threadIdx.x == 0) {
+      // vertices and degrees of everything found, spilled vertices included
+      // (kept ones: the edge slots handed out)
+      if (sm.few_n[par ^ 1]) atomicAdd(&back->n, (unsigned long long)sm.few_n[par ^ 1]);
+      const unsigned long long tot = sm.few_m[par ^ 1] + sm.few_edges[par ^ 1];
+      if (tot) atomicAdd(&back->m, tot);
+      if (blockIdx.x == 0) {
+        FewState& st = ctl->state;
+        st.L = L;
+        st.vis_n = ls.vis_n;
+        st.vis_m = ls.vis_m;
+        st.ps = ls.ps;
+        for (int k = 0; k < 8; ++k) st.mlp_raw[k] = sm.mlp_cache_raw[k];
+        st.mlp_margin = sm.mlp_cache_margin;
+        st.mlp_dec = sm.mlp_cache_dec;
+        // the ring descriptors and heavy counters start empty again, once
+        // every waiting CTA has read the level that the run began with
+        sm.waiting += nb - (unsigned)N;
+        unsigned long long t0 = 0;
+        uint32_t spins = 0;
+        while ((int)(ld_acquire_u32(&ctl->waiting) - sm.waiting) < 0) {
+          if ((++spins & 1023u) == 0) {
+            if (t0 == 0) t0 = globaltimer_ns();
+            if (globaltimer_ns() - t0 > p.timeout_ns) {
+              atomicCAS(&ctl->bar.err, 0, (int)XBFS_ERR_DEVICE_TIMEOUT);
+              break;
+            }
+          }
+        }
+        for (int i = 0; i < 4; ++i)
+          for (int k = 0; k < 8; ++k) reinterpret_cast<unsigned long long*>(&ctl->fd[i])[k] = 0ull;
+        ctl->heavy[0] = ctl->heavy[1] = 0ull;
+      }
+    }
+    if (!grid_sync(&ctl->bar, nb, epoch, p.timeout_ns)) return false;
+  }
+  if (threadIdx.x == 0) {
+    const volatile FewState* st = &ctl->state;
+    ls.vis_n = st->vis_n;
+    ls.vis_m = st->vis_m;
+    ls.ps.count_prev = st->ps.count_prev;
+    ls.ps.is_change = st->ps.is_change;
+    ls.ps.td_adaptive = st->ps.td_adaptive;
+    ls.ps.hub_before = st->ps.hub_before;
+    ls.ps.hub_after = st->ps.hub_after;
+    ls.ps.tag_prev = st->ps.tag_prev;
+    ls.ps.bu_dir = st->ps.bu_dir;
+    ls.ps.n_prev = st->ps.n_prev;
+    ls.ps.prev_strategy = st->ps.prev_strategy;
+    for (int k = 0; k < 8; ++k) sm.mlp_cache_raw[k] = st->mlp_raw[k];
+    sm.mlp_cache_margin = st->mlp_margin;
+    sm.mlp_cache_dec = st->mlp_dec;
+    sm.red4[0] = st->L;
+  }
+  __syncthreads();
+  return true;
+}
+
 // ---------------------------------------------------------------------------
 // The persistent traversal kernel.
 // ---------------------------------------------------------------------------
-template <bool PAR>
-__global__ void __launch_bounds__(kBlock, 2) k_bfs(Params p) {
+template <bool PAR, bool LEARNED>
+__global__ void __launch_bounds__(kBlock, 2) k_bfs(const __grid_constant__ Params p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   Ctl* ctl = p.ctl;
   if (p.absent_block > 0 && (int)blockIdx.x == p.absent_block - 1) return;  // test hook: never arrives
   if (threadIdx.x < 3) sm.cnt[threadIdx.x] = 0;
-  if (p.policy == XBFS_POLICY_MLP && p.mlp) mlp_stage(p.mlp, sm.mlp_w);
+  if (LEARNED) mlp_stage(p.mlp, sm.mlp_w);
   if (threadIdx.x == 0) sm.mlp_cache_dec = -1;
   __syncthreads();
 
@@ -2201,7 +2882,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(Params p) {
   // inner loop of the level.
   LoopState& ls = sm.ls;
   if (threadIdx.x == 0) {
-    if (p.policy == XBFS_POLICY_MLP && p.mlp) {
+    if (LEARNED) {
       // the installed bound after the weights, over each feature's scale
       const float* sd = sm.mlp_w + 8;
       const float* P = sm.mlp_w + kMlpParams;
@@ -2238,6 +2919,12 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(Params p) {
   const uint32_t nb = gridDim.x;
   uint32_t epoch = 0;
   long long L = 0;
+  unsigned runs = 0;        // runs of small levels so far
+  bool from_run = false;    // level L's frontier was handed back by one
+  if (threadIdx.x == 0) {
+    sm.waiting = 0;
+    sm.fitted = 0;
+  }
   if (p.fresh) {
     init_traversal<PAR>(p);
     if (!grid_sync(&ctl->bar, nb, epoch, p.timeout_ns)) return;
@@ -2274,7 +2961,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(Params p) {
       if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(&ctl->bar.err, 0, (int)XBFS_ERR_INTERNAL);
       break;
     }
-    FDesc* F0 = &ctl->fd[L & 3];
+    FDesc* F0 = from_run ? &ctl->back[(runs - 1) % 3] : &ctl->fd[L & 3];
     FDesc* F1 = &ctl->fd[(L + 1) & 3];
     FDesc* F2 = &ctl->fd[(L + 2) & 3];
     FDesc* F3 = &ctl->fd[(L + 3) & 3];
@@ -2301,6 +2988,18 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(Params p) {
       }
       sm.pend_next = pn;
       sm.spec = m_f <= kSpecEdges ? 1 : 0;
+      // CTAs for a run of small levels: few edges, none of the frontier in the
+      // larger bins, no early entries in the next one
+      sm.few = 0;
+      if ((unsigned long long)m_f <= (unsigned long long)(kFew * kFewShare) && pn == 0 &&
+          (sm.bins[0] & kCountMask) != 0 && ((sm.bins[1] | sm.bins[2]) & kCountMask) == 0) {
+        if (++sm.fitted > kFewAfter && p.small_max <= kFewEdges - kFewShare) {
+          const unsigned M = (unsigned)(sm.bins[0] >> 31), N = min((unsigned)kFew, gridDim.x);
+          if (M <= N * kFewShare) sm.few = M <= (unsigned)kSoloIn ? 1 : (int)N;
+        }
+      } else {
+        sm.fitted = 0;
+      }
       int s = -1;
       if (n_f > 0) {
         ls.vis_n += n_f;
@@ -2318,31 +3017,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(Params p) {
         sm.asyncq_ok = (n_u * 4 < p.V) ? 1 : 0;
         sm.mark_ok = (n_u * XBFS_MARK_NU_DIV >= p.V && m_f * 2 >= p.V) ? 1 : 0;
         sm.qside_ok = (n_u * 64 <= p.V && (pn == 0 || ls.pend_q_for == L + 1)) ? 1 : 0;
-        switch (p.policy) {
-          case XBFS_POLICY_FORCED: {
-            const long long i = L < p.n_forced ? L : p.n_forced - 1;
-            s = (i >= 0) ? (int)p.forced[i] : XBFS_TD_QUEUE;
-            if (s < 0 || s > 2) s = XBFS_TD_QUEUE;
-            break;
-          }
-          case XBFS_POLICY_BEAMER:
-            s = decide_beamer(ls.ps, n_f, m_f, m_u, p.V, p.beamer_alpha, p.beamer_beta);
-            break;
-          case XBFS_POLICY_MLP: {
-            const float raw[8] = {(float)n_f, (float)m_f, (float)n_u, (float)m_u, (float)L,
-                                  (float)ls.ps.prev_strategy, (float)ls.ps.n_prev, (float)m_f / (float)n_f};
-            if (sm.mlp_cache_dec >= 0 && mlp_reuse_bound(raw, sm.mlp_cache_raw, sm.mlp_q) < sm.mlp_cache_margin) {
-              s = sm.mlp_cache_dec;  // certified: the network would choose the same
-            } else {
-              s = -2;  // decided by warp 0 below
-#pragma unroll
-              for (int k = 0; k < 8; ++k) sm.mlp_raw[k] = raw[k];
-            }
-            break;
-          }
-          default:
-            s = decide_reference(ls.ps, L, m_f, p.E, p.alpha);
-        }
+        s = LEARNED ? decide_learned(sm, L, n_f, m_f, n_u, m_u) : decide(p, ls.ps, L, n_f, m_f, m_u);
         if (s == XBFS_BU && !p.allow_bu) s = XBFS_TD_QUEUE;
         if (blockIdx.x == 0 && L < p.hist_cap) {
           LevelRecDev& r = p.hist[L];
@@ -2359,13 +3034,12 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(Params p) {
       sm.strategy = s;
     }
     __syncthreads();
-    if (sm.strategy == -2) {
+    if (LEARNED && sm.strategy == -2) {
       // the learned switch: warp 0 evaluates it while the block waits (one
       // warp keeps the shared-memory and shuffle traffic of the network small)
       if (threadIdx.x < 32) {
-        int s2 = p.mlp ? mlp_decide(sm.mlp_w, sm.mlp_raw, threadIdx.x, sm.mlp_cache_raw, &sm.mlp_cache_dec,
-                                    &sm.mlp_cache_margin)
-                       : XBFS_TD_QUEUE;
+        int s2 = mlp_decide(sm.mlp_w, sm.mlp_raw, sm.mlp_act, threadIdx.x, sm.mlp_cache_raw, &sm.mlp_cache_dec,
+                            &sm.mlp_cache_margin);
         if (s2 == XBFS_BU && !p.allow_bu) s2 = XBFS_TD_QUEUE;
         if (threadIdx.x == 0) sm.strategy = s2;
       }
@@ -2373,6 +3047,22 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(Params p) {
     }
     const int S = sm.strategy;
     if (S < 0) break;  // empty frontier: done
+    // Few edges, all in the small bin, queue in and queue out: a few CTAs run
+    // this level and those after it (not in stepped launches, whose levels
+    // are timed one by one)
+    const bool small = p.fresh && S == XBFS_TD_QUEUE && q_valid && sm.few != 0;
+    from_run = false;
+    if (small) {
+      if (!small_levels<PAR, LEARNED>(p, sm, L, epoch, dirty, runs)) break;
+      ++epoch;
+      ++runs;
+      from_run = true;
+      b_valid = false;
+      dirty = 0;
+      L = sm.red4[0] - 1;  // the loop goes on at the level the run ended before
+      __syncthreads();
+      continue;
+    }
     if (threadIdx.x == 0) {
       ls.ps.prev_strategy = S;
       if (blockIdx.x == 0) {
@@ -2613,6 +3303,14 @@ static xbfs_status ensure_workspace(Graph* g, int small_max, int medium_max) {
   return XBFS_OK;
 }
 
+// The traversal kernel with or without parents and the learned switch. The
+// switch has a kernel of its own: its code in the others' would cost them 3 to
+// 4% on small graphs (R-MAT scale 16: 74.4 against 71.8 us).
+static const void* bfs_kernel(bool parents, bool learned) {
+  if (learned) return parents ? (const void*)k_bfs<true, true> : (const void*)k_bfs<false, true>;
+  return parents ? (const void*)k_bfs<true, false> : (const void*)k_bfs<false, false>;
+}
+
 // Fills the kernel parameters for one traversal of g with options o.
 static xbfs_status setup_params(Graph* g, const xbfs_opts& o, int* d_levels, int* d_parents, Params& p,
                                 const void** kfn_out, size_t* smem_out, int* grid_out) {
@@ -2662,7 +3360,7 @@ static xbfs_status setup_params(Graph* g, const xbfs_opts& o, int* d_levels, int
   p.allow_bu = g->symmetric ? 1 : 0;
 
   const bool par_on = d_parents != nullptr;
-  const void* kfn = par_on ? (const void*)k_bfs<true> : (const void*)k_bfs<false>;
+  const void* kfn = bfs_kernel(par_on, p.policy == XBFS_POLICY_MLP);
   // the weight copy of the learned switch sits at the end of Smem and is only
   // allocated for launches that use it (shared memory taken from L1)
   const size_t smem = sizeof(Smem) - (p.policy == XBFS_POLICY_MLP ? 0 : sizeof(((Smem*)0)->mlp_w));
@@ -3122,7 +3820,7 @@ xbfs_status level_costs(Graph* g, int32_t src, int32_t follow, int32_t cap, floa
 //   bits    5 * nw * 4      visited + 4 frontier bitmaps   cleared every call
 //   ctl     sizeof(Ctl)     barrier, descriptors, counters cleared every call
 //   rs      sizeof(ResumeState)                            unused (no stepping)
-//   ulist   nw * 32 * 4     bottom-up vertex lists         written before read
+//   ulist   V, to 32, * 4   bottom-up vertex lists         written before read
 //   heavy   3 arrays, (vertices of degree > 16) + 1 each   written before read
 //   queues  2 parities x 3 bins x (cap + 1) x (4 + 4 + 8)  written before read
 //   forced  n_forced bytes (forced policy only)            copied every call
@@ -3158,17 +3856,16 @@ xbfs_status noalloc_setup(int device, NoallocDevice** out) {
   if (!d.ready) {
     int nsm = 0;
     XBFS_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-    const void* fns[2] = {(const void*)k_bfs<false>, (const void*)k_bfs<true>};
-    for (int i = 0; i < 2; ++i) {
-      XBFS_CUDA_TRY(cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
+    for (int i = 0; i < 2; ++i)
       for (int m = 0; m < 2; ++m) {
+        const void* fn = bfs_kernel(i != 0, m != 0);
+        XBFS_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
         int per_sm = 0;
         XBFS_CUDA_TRY(
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fns[i], kBlock, m ? sizeof(Smem) : kSmemNoMlp));
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBlock, m ? sizeof(Smem) : kSmemNoMlp));
         if (per_sm < 1) return set_error(XBFS_ERR_INTERNAL, "traversal kernel cannot be resident");
         d.grid[i][m] = nsm * per_sm;
       }
-    }
     d.ready = true;
   }
   *out = &d;
@@ -3263,7 +3960,7 @@ xbfs_status bfs_noalloc(Graph* g, int32_t src, int32_t* levels, int32_t* parents
   const size_t o_bits = take(nw * 4 * 5);
   const size_t o_ctl = take(sizeof(Ctl));
   const size_t o_rs = take(sizeof(ResumeState));
-  const size_t o_ulist = take(nw * 32 * 4);
+  const size_t o_ulist = take((nw - 64) * 32 * 4);
   const size_t o_hid = take(hcap * 4), o_heb = take(hcap * 4), o_hbg = take(hcap * 8);
   size_t o_q[2][3][3];
   for (int par = 0; par < 2; ++par)
@@ -3330,7 +4027,7 @@ xbfs_status bfs_noalloc(Graph* g, int32_t src, int32_t* levels, int32_t* parents
   p.resume = 0;
   const bool par_on = parents != nullptr;
   const bool mlp_on = p.policy == XBFS_POLICY_MLP;
-  const void* kfn = par_on ? (const void*)k_bfs<true> : (const void*)k_bfs<false>;
+  const void* kfn = bfs_kernel(par_on, mlp_on);
   const size_t smem = mlp_on ? sizeof(Smem) : kSmemNoMlp;
   int grid = dev->grid[par_on ? 1 : 0][mlp_on ? 1 : 0];
   if (o.grid_dim > 0 && o.grid_dim < grid) grid = o.grid_dim;

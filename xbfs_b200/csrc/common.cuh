@@ -34,6 +34,14 @@ __device__ __forceinline__ uint64_t ld_acquire_u64(const unsigned long long* p) 
 __device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v) {
   asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+__device__ __forceinline__ uint64_t ld_relaxed_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 // Relaxed (weak, L2-coherent) load: bypasses L1 so a value written by another
 // SM earlier in the same persistent launch is observed once it reached L2.
 __device__ __forceinline__ uint32_t ld_cg_u32(const uint32_t* p) {
@@ -121,8 +129,13 @@ __device__ __forceinline__ void red_add_release_u32(uint32_t* p, uint32_t v) {
 // load that returns the arrival count and the error word together, so the
 // barrier costs one release and the polls, with no separate fence or status
 // read. 2^32 arrivals allow > 10^7 barriers at 296 CTAs.
+//
+// `progress` (optional) is a word that whoever the others wait for keeps
+// changing: the time limit then runs from its last change, and the poll is
+// slower from the start.
 __device__ __forceinline__ bool grid_sync(GridBarrier* bar, uint32_t nblocks, uint32_t& epoch,
-                                          unsigned long long timeout_ns) {
+                                          unsigned long long timeout_ns,
+                                          const unsigned long long* progress = nullptr) {
   __shared__ int s_ok;
   __syncthreads();
   epoch += 1;
@@ -131,7 +144,7 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* bar, uint32_t nblocks, ui
     const uint32_t target = epoch * nblocks;
     red_add_release_u32(&bar->count, 1u);
     uint32_t spins = 0;
-    unsigned long long t0 = 0;
+    unsigned long long t0 = 0, seen = 0;
     for (;;) {
       const unsigned long long w = ld_acquire_u64(reinterpret_cast<const unsigned long long*>(bar));
       if ((int32_t)(w >> 32) != 0) {
@@ -140,9 +153,14 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* bar, uint32_t nblocks, ui
       }
       if ((int32_t)((uint32_t)w - target) >= 0) break;
       ++spins;
-      if (spins > 2048) __nanosleep(32);
+      if (progress || spins > 2048) __nanosleep(progress ? 100 : 32);
       if ((spins & 1023u) == 0) {
         if (t0 == 0) t0 = globaltimer_ns();
+        if (progress) {
+          const unsigned long long now = ld_cg_u64(progress);
+          if (now != seen) t0 = globaltimer_ns();
+          seen = now;
+        }
         if (globaltimer_ns() - t0 > timeout_ns) {
           atomicCAS(&bar->err, 0, (int)XBFS_ERR_DEVICE_TIMEOUT);
           ok = 0;
