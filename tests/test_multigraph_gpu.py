@@ -79,3 +79,25 @@ def test_graph_larger_than_shared_bitmaps():
     mg = MultiGraph([Graph.from_csr(b, c) for b, c in cpu])
     srcs = pick(cpu, 1)
     check(mg, cpu, srcs, mg.bfs(srcs))
+
+
+@pytest.mark.parametrize("block,thread_max,alpha", [(256, 0, 4.0), (512, 32, 4.0), (1024, 8, 14.0),
+                                                    (512, 32, 0.001), (512, 100000, 1e9)])
+def test_graphs_shared_by_several_ctas(block, thread_max, alpha):
+    """Sets that mix graphs on both sides of the size at which several CTAs share
+    one: more of them than teams, lists above and below the length the team
+    shares, a frontier bitmap too large for shared memory, two components."""
+    cpu = [gen_rmat_host(int(11 + i % 5), 8 + i % 25, 40 + i) for i in range(45)]
+    cpu += [gen_er_host(14000 + 37 * i, 8.0, 90 + i) for i in range(6)]
+    cpu += [gen_er_host(800001, 3.0, 7)]
+    n = 70001  # star of 1025 and 60000 leaves, joined to nothing else but each other
+    pairs = np.array([(0, i) for i in range(2, 1027)] + [(1, i) for i in range(1000, 61000)], dtype=np.int64)
+    e = np.concatenate([pairs, pairs[:, ::-1]])
+    e = e[np.lexsort((e[:, 1], e[:, 0]))]
+    beg = np.concatenate([[0], np.cumsum(np.bincount(e[:, 0], minlength=n))]).astype(np.int64)
+    cpu += [(beg, e[:, 1].astype(np.int32)), gen_rmat_host(6, 8, 1)]
+    mg = MultiGraph([Graph.from_csr(b, c) for b, c in cpu])
+    mg.set_config(block, thread_max, alpha)
+    for seed in (1, 2):
+        srcs = pick(cpu, seed)
+        check(mg, cpu, srcs, mg.bfs(srcs))

@@ -3,15 +3,19 @@
 //
 // No counterpart in the reference (one graph per process). B200 design:
 //  * All graphs live in one arena (offsets per graph); a work list sorted by
-//    edge count (largest first) is consumed by CTAs through an atomic ticket,
-//    so the big graphs start first and the small ones fill the gaps
+//    edge count (largest first) is consumed through an atomic ticket, so the
+//    big graphs start first and the small ones fill the gaps
 //    (longest-processing-time order).
-//  * One CTA owns one graph for its whole traversal: visited / current /
-//    next frontier bitmaps sit in shared memory when V fits (up to 2^18
-//    vertices at 3 x 32 KB), so every status probe is a shared-memory access
-//    and levels are separated by __syncthreads instead of grid barriers.
-//    Larger graphs use a per-CTA slice of global scratch for the bitmaps.
-//  * Each level picks top-down or bottom-up from CTA-local counts. Top-down
+//  * Graphs of more than kBig vertices and edges are taken by teams of kTeam
+//    CTAs: bitmaps in global memory (L2), levels separated by a barrier of the
+//    team, the frontier copied to every CTA's shared memory for bottom-up
+//    probes, vertices of long lists shared by the whole team. When no such
+//    graph is left, the CTAs of a team go on singly.
+//  * Each other graph is owned by one CTA for its whole traversal: visited /
+//    current / next frontier bitmaps sit in shared memory (3 x 32 KB), so every
+//    status probe is a shared-memory access and levels are separated by
+//    __syncthreads.
+//  * Each level picks top-down or bottom-up from its own counts. Top-down
 //    expands frontier vertices of degree <= `thread_max` one per lane and
 //    heavier ones warp-cooperatively; bottom-up gives each lane one unvisited
 //    vertex and stops at the first parent.
@@ -32,6 +36,21 @@ namespace xbfs {
 
 namespace mg {
 
+// CTAs per team, and the vertices plus edges above which a graph is a team's.
+constexpr int kTeam = 8;
+constexpr long long kBig = 1 << 17;
+constexpr int kHeavy = 1024;  // a team shares the edges of vertices above this degree
+constexpr unsigned long long kTimeoutNs = 10ull * 1000 * 1000 * 1000;
+
+// One team's state. Counters are rings by level: a level reads its own slot,
+// adds to the next one and clears the one after that.
+struct Team {
+  GridBarrier bar;
+  int graph;                    // ticket drawn for the team
+  unsigned heavy[4];            // length of the list of long vertices
+  unsigned long long n[4], m[4];  // frontier vertices, degree sum
+};
+
 struct Desc {
   long long b_off;   // offset of the graph's V+1 local offsets in the beg arena
   long long e_off;   // offset of its neighbours in the csr arena
@@ -49,8 +68,13 @@ struct Params {
   int n;
   int* levels;            // concatenated outputs
   unsigned* ticket;
-  uint32_t* gscratch;     // per-CTA global bitmaps for graphs too large for shared memory
-  long long gscratch_words;  // words per CTA (3 bitmaps)
+  int n_big;              // the first n_big graphs of `order` are the teams'
+  Team* teams;
+  uint32_t* bits;         // per team: visited and three frontier bitmaps of team_words words
+  long long team_words;
+  int* heavy;             // per team: list of long vertices, heavy_cap entries
+  long long heavy_cap;
+  int* err;               // status of the launch
   int smem_words;         // words per bitmap available in shared memory
   int thread_max;         // top-down: degree <= thread_max expanded by one lane
   float alpha;            // bottom-up when m_f * alpha > m_u
@@ -62,16 +86,237 @@ __device__ __forceinline__ long long block_sum_ll(long long v, long long* red) {
   return block_sum<BLOCK, long long>(v, red);
 }
 
+// One claimed edge of a team's top-down level.
+__device__ __forceinline__ void team_claim(uint32_t* vis, uint32_t* nxt, const long long* beg, int* lv, int v, int level,
+                                           long long& n, long long& m) {
+  const uint32_t bit = 1u << (v & 31);
+  if (ld_cg_u32(vis + (v >> 5)) & bit) return;
+  if (atomicOr(vis + (v >> 5), bit) & bit) return;
+  red_or_u32(nxt + (v >> 5), bit);
+  lv[v] = level;
+  n += 1;
+  m += __ldg(beg + v + 1) - __ldg(beg + v);
+}
+
+// Four edges of a lane, their targets read together.
+__device__ __forceinline__ void team_claim4(const int* csr, long long e, long long step, long long e1, uint32_t* vis,
+                                            uint32_t* nxt, const long long* beg, int* lv, int level, long long& n,
+                                            long long& m) {
+  int v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] = e + k * step < e1 ? __ldg(csr + e + k * step) : -1;
+  uint32_t w[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) w[k] = v[k] >= 0 ? ld_cg_u32(vis + (v[k] >> 5)) : ~0u;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (v[k] >= 0 && !((w[k] >> (v[k] & 31)) & 1u)) team_claim(vis, nxt, beg, lv, v[k], level, n, m);
+}
+
+// One graph by a team of kTeam CTAs (rank: this CTA's place in it). False:
+// the time limit of a barrier ran out.
+template <int BLOCK>
+__device__ bool team_bfs(const Params& p, Team* team, uint32_t* bits, int* heavy, int rank, uint32_t& epoch, int gi,
+                         uint32_t* sbits, long long* red, int* s_decision, long long* s_mu) {
+  constexpr int NW = BLOCK / 32;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const Desc d = p.desc[p.order[gi]];
+  const long long* beg = p.beg + d.b_off;
+  const int* csr = p.csr + d.e_off;
+  int* lv = p.levels + d.v_off;
+  const int nw = (d.V + 31) / 32;
+  uint32_t* vis = bits;
+  uint32_t* fr[3] = {bits + p.team_words, bits + 2 * p.team_words, bits + 3 * p.team_words};
+  const int src = d.src;
+  // CTA ranks take words in turn, a warp's worth of words each (all of them
+  // see dense and sparse parts of the vertex range)
+  const int gw = wid * kTeam + rank;       // this warp among the team's
+  constexpr int GW = NW * kTeam;
+  for (int w = rank * BLOCK + threadIdx.x; w < nw; w += kTeam * BLOCK) {
+    const uint32_t own = (w == (src >> 5)) ? 1u << (src & 31) : 0u;
+    vis[w] = own | ((w == nw - 1 && (d.V & 31)) ? ~((1u << (d.V & 31)) - 1u) : 0u);
+    fr[0][w] = own;
+    fr[1][w] = 0u;
+    fr[2][w] = 0u;
+  }
+  if (rank == 0 && threadIdx.x == 0) {
+    lv[src] = 0;
+    team->n[0] = 1ull;
+    team->m[0] = (unsigned long long)(beg[src + 1] - beg[src]);
+    for (int k = 1; k < 4; ++k) team->n[k] = team->m[k] = 0ull;
+    for (int k = 0; k < 4; ++k) team->heavy[k] = 0u;
+  }
+  if (threadIdx.x == 0) *s_mu = d.E;
+  if (!grid_sync(&team->bar, kTeam, epoch, kTimeoutNs)) return false;
+  unsigned long long reached = 0;  // thread 0 of rank 0
+  for (int L = 0;; ++L) {
+    if (threadIdx.x == 0) {
+      const long long n_f = (long long)ld_cg_u64(&team->n[L & 3]), m_f = (long long)ld_cg_u64(&team->m[L & 3]);
+      *s_mu -= m_f;
+      reached += (unsigned long long)m_f;
+      *s_decision = n_f == 0 ? -1 : ((double)m_f * (double)p.alpha > (double)*s_mu ? 1 : 0);
+      if (rank == 0) {
+        team->n[(L + 2) & 3] = team->m[(L + 2) & 3] = 0ull;
+        team->heavy[(L + 2) & 3] = 0u;
+      }
+    }
+    __syncthreads();
+    const int dec = *s_decision;
+    if (dec < 0) break;
+    const uint32_t* cur = fr[L % 3];
+    uint32_t* nxt = fr[(L + 1) % 3];
+    uint32_t* old = fr[(L + 2) % 3];
+    long long my_n = 0, my_m = 0;
+    // frontier L-1's bitmap becomes frontier L+2's
+    for (int w = rank * BLOCK + threadIdx.x; w < nw; w += kTeam * BLOCK) old[w] = 0u;
+    if (dec == 1) {
+      // ---- bottom-up over the frontier's bitmap in shared memory
+      const bool staged = nw <= 3 * p.smem_words;
+      if (staged) {
+        for (int w = threadIdx.x; w < nw; w += BLOCK) sbits[w] = ld_cg_u32(cur + w);
+        __syncthreads();
+      }
+      const uint32_t* f = staged ? sbits : cur;
+      for (int w = gw; w < nw; w += GW) {
+        const uint32_t un = ~ld_cg_u32(vis + w);
+        if (!un) continue;
+        const int v = w * 32 + lane;
+        bool found = false, more = false;
+        long long e0 = 0, e1 = 0;
+        if ((un >> lane) & 1u) {
+          e0 = __ldg(beg + v);
+          e1 = __ldg(beg + v + 1);
+          const long long d0 = e1 - e0;
+          // up to eight neighbours by the lane itself, four at a time
+          for (long long e = e0; e < e1 && e < e0 + 8 && !found; e += 4) {
+            int u[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) u[k] = e + k < e1 ? __ldg(csr + e + k) : -1;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) found = found || (u[k] >= 0 && ((f[u[k] >> 5] >> (u[k] & 31)) & 1u));
+          }
+          more = !found && d0 > 8;
+          e0 += 8;
+        }
+        // the rest of the longer lists by the whole warp, one after another
+        unsigned rest = __ballot_sync(0xffffffffu, more);
+        while (rest) {
+          const int hl = __ffs(rest) - 1;
+          rest &= rest - 1;
+          const long long h1 = __shfl_sync(0xffffffffu, e1, hl);
+          for (long long e = __shfl_sync(0xffffffffu, e0, hl); e < h1; e += 64) {
+            bool hit = false;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const long long x = e + k * 32 + lane;
+              const int u = x < h1 ? __ldg(csr + x) : -1;
+              hit = hit || (u >= 0 && ((f[u >> 5] >> (u & 31)) & 1u));
+            }
+            if (__any_sync(0xffffffffu, hit)) {
+              if (lane == hl) found = true;
+              break;
+            }
+          }
+        }
+        if (found) {
+          lv[v] = L + 1;
+          my_n += 1;
+          my_m += __ldg(beg + v + 1) - __ldg(beg + v);
+        }
+        const unsigned got = __ballot_sync(0xffffffffu, found);
+        if (lane == 0 && got) {
+          nxt[w] = got;
+          vis[w] = ~un | got;
+        }
+      }
+      __syncthreads();
+    } else {
+      // ---- top-down
+      unsigned* hc = &team->heavy[L & 3];
+      for (int w = gw; w < nw; w += GW) {
+        const uint32_t mine_bits = ld_cg_u32(cur + w);
+        if (!mine_bits) continue;
+        const int u = w * 32 + lane;
+        const bool mine = (mine_bits >> lane) & 1u;
+        long long e0 = 0, e1 = 0;
+        if (mine) {
+          e0 = __ldg(beg + u);
+          e1 = __ldg(beg + u + 1);
+        }
+        const long long deg = e1 - e0;
+        if (mine && deg <= p.thread_max)
+          for (long long e = e0; e < e1; e += 4) team_claim4(csr, e, 1, e1, vis, nxt, beg, lv, L + 1, my_n, my_m);
+        if (mine && deg > p.thread_max && deg > kHeavy) {
+          const unsigned at = atomicAdd(hc, 1u);
+          heavy[at] = u;
+        }
+        unsigned mid = __ballot_sync(0xffffffffu, mine && deg > p.thread_max && deg <= kHeavy);
+        while (mid) {
+          const int hl = __ffs(mid) - 1;
+          mid &= mid - 1;
+          const long long h0 = __shfl_sync(0xffffffffu, e0, hl), h1 = __shfl_sync(0xffffffffu, e1, hl);
+          for (long long e = h0 + lane; e < h1; e += 128)
+            team_claim4(csr, e, 32, h1, vis, nxt, beg, lv, L + 1, my_n, my_m);
+        }
+      }
+      if (!grid_sync(&team->bar, kTeam, epoch, kTimeoutNs)) return false;
+      const unsigned nh = ld_cg_u32(hc);
+      for (unsigned h = 0; h < nh; ++h) {
+        const int u = (int)ld_cg_u32(reinterpret_cast<const uint32_t*>(heavy + h));
+        const long long h0 = __ldg(beg + u), h1 = __ldg(beg + u + 1);
+        constexpr long long step = (long long)kTeam * BLOCK;
+        for (long long e = h0 + rank * BLOCK + threadIdx.x; e < h1; e += 4 * step)
+          team_claim4(csr, e, step, h1, vis, nxt, beg, lv, L + 1, my_n, my_m);
+      }
+    }
+    long long x[2] = {my_n, my_m};
+    block_sum_n<BLOCK, 2, long long>(x, red);
+    if (threadIdx.x == 0 && x[0]) {
+      atomicAdd(&team->n[(L + 1) & 3], (unsigned long long)x[0]);
+      atomicAdd(&team->m[(L + 1) & 3], (unsigned long long)x[1]);
+    }
+    if (!grid_sync(&team->bar, kTeam, epoch, kTimeoutNs)) return false;
+  }
+  if (rank == 0 && threadIdx.x == 0) p.edges[p.order[gi]] = reached;
+  __syncthreads();
+  return true;
+}
+
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_multi(Params p) {
   extern __shared__ __align__(16) uint32_t sbits[];
-  __shared__ long long red[BLOCK / 32 + 1];
+  __shared__ long long red[2 * (BLOCK / 32) + 1];
   __shared__ int s_g;
-  __shared__ unsigned long long s_nf, s_mf, s_mdone;
+  __shared__ long long s_mu;
+  __shared__ unsigned long long s_nf, s_mf;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   constexpr int NW = BLOCK / 32;
+  // ---- the teams' graphs: the team's first CTA draws the tickets
+  if (p.n_big > 0) {
+    const int t = blockIdx.x / kTeam, rank = blockIdx.x % kTeam;
+    Team* team = p.teams + t;
+    uint32_t epoch = 0;
+    bool ok = true;
+    for (;;) {
+      if (rank == 0 && threadIdx.x == 0) team->graph = (int)atomicAdd(p.ticket + 1, 1u);
+      ok = grid_sync(&team->bar, kTeam, epoch, kTimeoutNs);
+      if (!ok) break;
+      if (threadIdx.x == 0) s_g = ld_acquire_i32(&team->graph);
+      __syncthreads();
+      const int gi = s_g;
+      if (gi >= p.n_big) break;
+      ok = team_bfs<BLOCK>(p, team, p.bits + (size_t)t * 4 * p.team_words, p.heavy + (size_t)t * p.heavy_cap, rank,
+                           epoch, gi, sbits, red, &s_g, &s_mu);
+      if (!ok) break;
+    }
+    if (!ok) {
+      if (threadIdx.x == 0) atomicCAS(p.err, 0, (int)XBFS_ERR_DEVICE_TIMEOUT);
+      return;
+    }
+    __syncthreads();
+  }
   for (;;) {
-    if (threadIdx.x == 0) s_g = (int)atomicAdd(p.ticket, 1u);
+    if (threadIdx.x == 0) s_g = p.n_big + (int)atomicAdd(p.ticket, 1u);
     __syncthreads();
     const int gi = s_g;
     if (gi >= p.n) break;
@@ -81,19 +326,10 @@ __global__ void __launch_bounds__(BLOCK) k_multi(Params p) {
     const int* csr = p.csr + d.e_off;
     int* lv = p.levels + d.v_off;
     const int nw = (V + 31) / 32;
-    // volatile: on the global-scratch path a plain load could hit an L1 line
-    // made stale by another thread's atomic (atomics update L2 only)
-    volatile uint32_t *vis, *cur, *nxt;
-    if (nw <= p.smem_words) {
-      vis = sbits;
-      cur = sbits + p.smem_words;
-      nxt = sbits + 2 * p.smem_words;
-    } else {
-      uint32_t* base = p.gscratch + (size_t)blockIdx.x * p.gscratch_words;
-      vis = base;
-      cur = base + nw;
-      nxt = base + 2 * (size_t)nw;
-    }
+    // volatile: a word that another thread changes by an atomic is read anew
+    volatile uint32_t* vis = sbits;
+    volatile uint32_t* cur = sbits + p.smem_words;
+    volatile uint32_t* nxt = sbits + 2 * p.smem_words;
     for (int w = threadIdx.x; w < nw; w += BLOCK) {
       // bits past V count as visited so they are never searched
       const uint32_t tail = (w == nw - 1 && (V & 31)) ? ~((1u << (V & 31)) - 1u) : 0u;
@@ -214,11 +450,14 @@ struct MultiGraph {
   int device = 0;
   int n = 0;
   long long total_V = 0, total_E = 0;
-  int maxV = 0;
-  DevBuf beg, csr, desc, order, ticket, edges, gscratch, srcs_dev, levels_tmp;
+  int n_big = 0;                 // graphs for teams, first in `horder`
+  int max_teams = 0;             // teams the buffers are laid out for
+  long long team_words = 0, heavy_cap = 0;
+  size_t ctl_teams = 0;          // offset of the teams in ctl
+  DevBuf beg, csr, desc, order, ctl, bits, heavy, srcs_dev, levels_tmp;
   std::vector<mg::Desc> hdesc;
   std::vector<int> horder;
-  PinnedBuf srcs_pin;
+  PinnedBuf srcs_pin, ctl_pin;
   cudaStream_t stream = nullptr;
   // tuned configuration
   int block = 512;
@@ -239,15 +478,19 @@ struct MultiGraph {
   }
 };
 
-static int smem_words_for(int block) {
-  (void)block;
-  return 8192;  // 3 x 32 KB: graphs up to 262,144 vertices keep their bitmaps on chip
-}
+// 3 x 32 KB: a single CTA's bitmaps of up to 262,144 vertices (larger graphs
+// are the teams', as kBig is below that).
+constexpr int kSmemWords = 8192;
+static_assert(mg::kBig <= 32ll * kSmemWords, "graphs too large for shared memory must be the teams'");
+// Control buffer, cleared before every launch: two tickets (single CTAs,
+// teams) and the launch status; from kCtlEdges the graphs' edge counts; then
+// the teams. What lies before the teams is copied to the host after it.
+constexpr size_t kCtlEdges = 64;
 
 static xbfs_status enqueue_multi(MultiGraph* m, int* d_levels, int block, int thread_max, float alpha) {
   cudaStream_t s = m->stream;
   XBFS_CUDA_TRY(cudaMemsetAsync(d_levels, 0xff, (size_t)m->total_V * 4, s));
-  XBFS_CUDA_TRY(cudaMemsetAsync(m->ticket.p, 0, 16, s));
+  XBFS_CUDA_TRY(cudaMemsetAsync(m->ctl.p, 0, m->ctl.bytes, s));
   // the per-graph sources are patched into the descriptors on the device
   mg::Params p;
   p.beg = m->beg.as<long long>();
@@ -256,13 +499,18 @@ static xbfs_status enqueue_multi(MultiGraph* m, int* d_levels, int block, int th
   p.order = m->order.as<int>();
   p.n = m->n;
   p.levels = d_levels;
-  p.ticket = m->ticket.as<unsigned>();
-  p.gscratch = m->gscratch.as<uint32_t>();
-  p.gscratch_words = 3ll * ((m->maxV + 31) / 32);
-  p.smem_words = smem_words_for(block);
+  p.ticket = m->ctl.as<unsigned>();
+  p.err = m->ctl.as<int>() + 2;
+  p.teams = reinterpret_cast<mg::Team*>(m->ctl.as<char>() + m->ctl_teams);
+  p.n_big = m->n_big;
+  p.bits = m->bits.as<uint32_t>();
+  p.team_words = m->team_words;
+  p.heavy = m->heavy.as<int>();
+  p.heavy_cap = m->heavy_cap;
+  p.smem_words = kSmemWords;
   p.thread_max = thread_max;
   p.alpha = alpha;
-  p.edges = m->edges.as<unsigned long long>();
+  p.edges = reinterpret_cast<unsigned long long*>(m->ctl.as<char>() + kCtlEdges);
   const size_t smem = (size_t)3 * p.smem_words * 4;
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device);
@@ -276,9 +524,17 @@ static xbfs_status enqueue_multi(MultiGraph* m, int* d_levels, int block, int th
   int per_sm = 0;
   XBFS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, block, smem));
   if (per_sm < 1) return set_error(XBFS_ERR_INTERNAL, "multi-graph kernel cannot be resident");
-  const int grid = std::min(nsm * per_sm, m->n);
   void* args[] = {&p};
-  XBFS_CUDA_TRY(cudaLaunchKernel(kfn, dim3(grid), dim3(block), args, smem, s));
+  if (m->n_big > 0) {
+    // whole teams, all resident (their CTAs wait for one another); no more
+    // teams than can have work
+    const int single = (m->n - m->n_big + mg::kTeam - 1) / mg::kTeam;
+    const int teams = std::min({nsm * per_sm / mg::kTeam, m->n_big + single, m->max_teams});
+    if (teams < 1) return set_error(XBFS_ERR_INTERNAL, "multi-graph kernel cannot be resident");
+    XBFS_CUDA_TRY(cudaLaunchCooperativeKernel(kfn, dim3(teams * mg::kTeam), dim3(block), args, smem, s));
+  } else {
+    XBFS_CUDA_TRY(cudaLaunchKernel(kfn, dim3(std::min(nsm * per_sm, m->n)), dim3(block), args, smem, s));
+  }
   return XBFS_OK;
 }
 
@@ -310,6 +566,10 @@ static xbfs_status run_multi(MultiGraph* m, int* d_levels, int block, int thread
       }
       if (e != cudaSuccess) st = set_error(XBFS_ERR_CUDA, "capture: %s", cudaGetErrorString(e));
       if (!st) st = enqueue_multi(m, d_levels, block, thread_max, alpha);
+      if (!st) {
+        e = cudaMemcpyAsync(m->ctl_pin.p, m->ctl.p, m->ctl_teams, cudaMemcpyDeviceToHost, s);
+        if (e != cudaSuccess) st = set_error(XBFS_ERR_CUDA, "capture: %s", cudaGetErrorString(e));
+      }
     }
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
     if (st) {
@@ -332,6 +592,8 @@ static xbfs_status run_multi(MultiGraph* m, int* d_levels, int block, int thread
   float ms = 0;
   XBFS_CUDA_TRY(cudaEventElapsedTime(&ms, m->e0, m->e1));
   if (ms_out) *ms_out = ms;
+  const int err = m->ctl_pin.as<int>()[2];
+  if (err) return set_error((xbfs_status)err, "multi-graph kernel reported %s", xbfs_strerror(err));
   return XBFS_OK;
 }
 
@@ -360,14 +622,13 @@ xbfs_status xbfs_multi_create(xbfs_graph* const* graphs, int32_t n, int32_t devi
     vb += g->V;
     bb += g->V + 1;
     eb += g->E;
-    m->maxV = std::max<int>(m->maxV, (int)g->V);
   }
   m->total_V = vb;
   m->total_E = eb;
   xbfs_status st;
   if ((st = m->beg.ensure((size_t)bb * 8)) || (st = m->csr.ensure((size_t)eb * 4 + 64)) ||
       (st = m->desc.ensure(sizeof(mg::Desc) * n)) || (st = m->order.ensure(sizeof(int) * n)) ||
-      (st = m->ticket.ensure(16)) || (st = m->edges.ensure(8 * (size_t)n)) || (st = m->srcs_dev.ensure(4 * (size_t)n)) ||
+      (st = m->srcs_dev.ensure(4 * (size_t)n)) ||
       (st = m->srcs_pin.ensure(4 * (size_t)n)))
     return st;
   XBFS_CUDA_TRY(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
@@ -388,15 +649,29 @@ xbfs_status xbfs_multi_create(xbfs_graph* const* graphs, int32_t n, int32_t devi
   });
   XBFS_CUDA_TRY(cudaMemcpyAsync(m->desc.p, m->hdesc.data(), sizeof(mg::Desc) * n, cudaMemcpyHostToDevice, m->stream));
   XBFS_CUDA_TRY(cudaMemcpyAsync(m->order.p, m->horder.data(), sizeof(int) * n, cudaMemcpyHostToDevice, m->stream));
-  // global bitmap scratch only for graphs that do not fit the on-chip bitmaps
-  int nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-  const long long words = 3ll * ((m->maxV + 31) / 32);
-  if ((m->maxV + 31) / 32 > smem_words_for(256)) {
-    if ((st = m->gscratch.ensure((size_t)words * 4 * nsm * 8))) return st;
-  } else {
-    if ((st = m->gscratch.ensure(16))) return st;
+  // the teams' bitmaps and lists, for as many teams as a launch may have
+  long long big_v = 0, big_long = 0;
+  for (int i = 0; i < n; ++i) {
+    const mg::Desc& d = m->hdesc[i];
+    if (d.E + d.V <= mg::kBig) continue;
+    ++m->n_big;
+    big_v = std::max<long long>(big_v, d.V);
+    big_long = std::max<long long>(big_long, ((const Graph*)graphs[i])->cnt_deg_gt[10]);
   }
+  if (m->n_big > 0) {
+    int nsm = 148;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+    m->max_teams = std::max(1, nsm * 2 / mg::kTeam);  // shared memory admits two CTAs per SM
+    m->team_words = (big_v + 31) / 32;
+    m->heavy_cap = big_long + 1;
+    if ((st = m->bits.ensure((size_t)m->max_teams * 4 * (size_t)m->team_words * 4)) ||
+        (st = m->heavy.ensure((size_t)m->max_teams * (size_t)m->heavy_cap * 4)))
+      return st;
+  }
+  m->ctl_teams = (kCtlEdges + 8 * (size_t)n + 63) & ~(size_t)63;
+  if ((st = m->ctl.ensure(m->ctl_teams + sizeof(mg::Team) * (size_t)m->max_teams)) ||
+      (st = m->ctl_pin.ensure(m->ctl_teams)))
+    return st;
   XBFS_CUDA_TRY(cudaStreamSynchronize(m->stream));
   *out = (xbfs_multi*)m.release();
   return XBFS_OK;
@@ -433,12 +708,11 @@ xbfs_status xbfs_multi_bfs(xbfs_multi* mh, const int32_t* srcs, int32_t* levels,
   if ((st = run_multi(m, d_levels, m->block, m->thread_max, m->alpha, &ms))) return st;
   if (!dev) XBFS_CUDA_TRY(cudaMemcpy(levels, d_levels, (size_t)m->total_V * 4, cudaMemcpyDeviceToHost));
   if (stats) {
-    std::vector<unsigned long long> e(m->n);
-    XBFS_CUDA_TRY(cudaMemcpy(e.data(), m->edges.p, 8 * (size_t)m->n, cudaMemcpyDeviceToHost));
+    const unsigned long long* e = reinterpret_cast<unsigned long long*>(m->ctl_pin.as<char>() + kCtlEdges);
     memset(stats, 0, sizeof(*stats));
     stats->struct_size = (int32_t)sizeof(xbfs_stats);
     unsigned long long tot = 0;
-    for (auto x : e) tot += x / 2;
+    for (int i = 0; i < m->n; ++i) tot += e[i] / 2;
     stats->edges_mc = (int64_t)tot;
     stats->device_ms = ms;
     stats->kernel_ms = ms;
