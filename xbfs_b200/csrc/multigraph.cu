@@ -6,8 +6,8 @@
 //    edge count (largest first) is consumed through an atomic ticket, so the
 //    big graphs start first and the small ones fill the gaps
 //    (longest-processing-time order).
-//  * Graphs of more than kBig vertices and edges are taken by teams of kTeam
-//    CTAs: bitmaps in global memory (L2), levels separated by a barrier of the
+//  * Graphs of more than kBig vertices and edges are taken by teams of 8 to
+//    64 CTAs: bitmaps in global memory (L2), levels separated by a barrier of the
 //    team, the frontier copied to every CTA's shared memory for bottom-up
 //    probes, vertices of long lists shared by the whole team. When no such
 //    graph is left, the CTAs of a team go on singly.
@@ -36,8 +36,11 @@ namespace xbfs {
 
 namespace mg {
 
-// CTAs per team, and the vertices plus edges above which a graph is a team's.
-constexpr int kTeam = 8;
+// CTAs per team (at least, at most), and the vertices plus edges above which a
+// graph is a team's. Teams are as large as lets all big graphs run side by
+// side: 16 graphs (up to R-MAT scale 18) take 0.55 ms in teams of 8 and 0.36 in
+// teams of 16, 96 graphs 0.86 and 1.07.
+constexpr int kTeamMin = 8, kTeamMax = 64;
 constexpr long long kBig = 1 << 17;
 constexpr int kHeavy = 1024;  // a team shares the edges of vertices above this degree
 constexpr unsigned long long kTimeoutNs = 10ull * 1000 * 1000 * 1000;
@@ -69,6 +72,7 @@ struct Params {
   int* levels;            // concatenated outputs
   unsigned* ticket;
   int n_big;              // the first n_big graphs of `order` are the teams'
+  int team;               // CTAs per team
   Team* teams;
   uint32_t* bits;         // per team: visited and three frontier bitmaps of team_words words
   long long team_words;
@@ -113,7 +117,7 @@ __device__ __forceinline__ void team_claim4(const int* csr, long long e, long lo
     if (v[k] >= 0 && !((w[k] >> (v[k] & 31)) & 1u)) team_claim(vis, nxt, beg, lv, v[k], level, n, m);
 }
 
-// One graph by a team of kTeam CTAs (rank: this CTA's place in it). False:
+// One graph by a team of p.team CTAs (rank: this CTA's place in it). False:
 // the time limit of a barrier ran out.
 template <int BLOCK>
 __device__ bool team_bfs(const Params& p, Team* team, uint32_t* bits, int* heavy, int rank, uint32_t& epoch, int gi,
@@ -130,9 +134,10 @@ __device__ bool team_bfs(const Params& p, Team* team, uint32_t* bits, int* heavy
   const int src = d.src;
   // CTA ranks take words in turn, a warp's worth of words each (all of them
   // see dense and sparse parts of the vertex range)
-  const int gw = wid * kTeam + rank;       // this warp among the team's
-  constexpr int GW = NW * kTeam;
-  for (int w = rank * BLOCK + threadIdx.x; w < nw; w += kTeam * BLOCK) {
+  const int T = p.team;
+  const int gw = wid * T + rank;  // this warp among the team's
+  const int GW = NW * T;
+  for (int w = rank * BLOCK + threadIdx.x; w < nw; w += T * BLOCK) {
     const uint32_t own = (w == (src >> 5)) ? 1u << (src & 31) : 0u;
     vis[w] = own | ((w == nw - 1 && (d.V & 31)) ? ~((1u << (d.V & 31)) - 1u) : 0u);
     fr[0][w] = own;
@@ -147,7 +152,7 @@ __device__ bool team_bfs(const Params& p, Team* team, uint32_t* bits, int* heavy
     for (int k = 0; k < 4; ++k) team->heavy[k] = 0u;
   }
   if (threadIdx.x == 0) *s_mu = d.E;
-  if (!grid_sync(&team->bar, kTeam, epoch, kTimeoutNs)) return false;
+  if (!grid_sync(&team->bar, (uint32_t)p.team, epoch, kTimeoutNs)) return false;
   unsigned long long reached = 0;  // thread 0 of rank 0
   for (int L = 0;; ++L) {
     if (threadIdx.x == 0) {
@@ -168,7 +173,7 @@ __device__ bool team_bfs(const Params& p, Team* team, uint32_t* bits, int* heavy
     uint32_t* old = fr[(L + 2) % 3];
     long long my_n = 0, my_m = 0;
     // frontier L-1's bitmap becomes frontier L+2's
-    for (int w = rank * BLOCK + threadIdx.x; w < nw; w += kTeam * BLOCK) old[w] = 0u;
+    for (int w = rank * BLOCK + threadIdx.x; w < nw; w += T * BLOCK) old[w] = 0u;
     if (dec == 1) {
       // ---- bottom-up over the frontier's bitmap in shared memory
       const bool staged = nw <= 3 * p.smem_words;
@@ -259,12 +264,12 @@ __device__ bool team_bfs(const Params& p, Team* team, uint32_t* bits, int* heavy
             team_claim4(csr, e, 32, h1, vis, nxt, beg, lv, L + 1, my_n, my_m);
         }
       }
-      if (!grid_sync(&team->bar, kTeam, epoch, kTimeoutNs)) return false;
+      if (!grid_sync(&team->bar, (uint32_t)p.team, epoch, kTimeoutNs)) return false;
       const unsigned nh = ld_cg_u32(hc);
       for (unsigned h = 0; h < nh; ++h) {
         const int u = (int)ld_cg_u32(reinterpret_cast<const uint32_t*>(heavy + h));
         const long long h0 = __ldg(beg + u), h1 = __ldg(beg + u + 1);
-        constexpr long long step = (long long)kTeam * BLOCK;
+        const long long step = (long long)T * BLOCK;
         for (long long e = h0 + rank * BLOCK + threadIdx.x; e < h1; e += 4 * step)
           team_claim4(csr, e, step, h1, vis, nxt, beg, lv, L + 1, my_n, my_m);
       }
@@ -275,7 +280,7 @@ __device__ bool team_bfs(const Params& p, Team* team, uint32_t* bits, int* heavy
       atomicAdd(&team->n[(L + 1) & 3], (unsigned long long)x[0]);
       atomicAdd(&team->m[(L + 1) & 3], (unsigned long long)x[1]);
     }
-    if (!grid_sync(&team->bar, kTeam, epoch, kTimeoutNs)) return false;
+    if (!grid_sync(&team->bar, (uint32_t)p.team, epoch, kTimeoutNs)) return false;
   }
   if (rank == 0 && threadIdx.x == 0) p.edges[p.order[gi]] = reached;
   __syncthreads();
@@ -293,13 +298,13 @@ __global__ void __launch_bounds__(BLOCK) k_multi(Params p) {
   constexpr int NW = BLOCK / 32;
   // ---- the teams' graphs: the team's first CTA draws the tickets
   if (p.n_big > 0) {
-    const int t = blockIdx.x / kTeam, rank = blockIdx.x % kTeam;
+    const int t = blockIdx.x / p.team, rank = blockIdx.x % p.team;
     Team* team = p.teams + t;
     uint32_t epoch = 0;
     bool ok = true;
     for (;;) {
       if (rank == 0 && threadIdx.x == 0) team->graph = (int)atomicAdd(p.ticket + 1, 1u);
-      ok = grid_sync(&team->bar, kTeam, epoch, kTimeoutNs);
+      ok = grid_sync(&team->bar, (uint32_t)p.team, epoch, kTimeoutNs);
       if (!ok) break;
       if (threadIdx.x == 0) s_g = ld_acquire_i32(&team->graph);
       __syncthreads();
@@ -461,8 +466,9 @@ struct MultiGraph {
   cudaStream_t stream = nullptr;
   // tuned configuration
   int block = 512;
-  int thread_max = 32;
-  float alpha = 4.f;
+  // before tuning; with 8 and 14 the 96-graph set takes 0.86 ms, with 32 and 4 1.40
+  int thread_max = 8;
+  float alpha = 14.f;
   // captured replay
   cudaGraphExec_t exec = nullptr;
   int* exec_levels = nullptr;
@@ -503,6 +509,7 @@ static xbfs_status enqueue_multi(MultiGraph* m, int* d_levels, int block, int th
   p.err = m->ctl.as<int>() + 2;
   p.teams = reinterpret_cast<mg::Team*>(m->ctl.as<char>() + m->ctl_teams);
   p.n_big = m->n_big;
+  p.team = 1;
   p.bits = m->bits.as<uint32_t>();
   p.team_words = m->team_words;
   p.heavy = m->heavy.as<int>();
@@ -528,10 +535,13 @@ static xbfs_status enqueue_multi(MultiGraph* m, int* d_levels, int block, int th
   if (m->n_big > 0) {
     // whole teams, all resident (their CTAs wait for one another); no more
     // teams than can have work
-    const int single = (m->n - m->n_big + mg::kTeam - 1) / mg::kTeam;
-    const int teams = std::min({nsm * per_sm / mg::kTeam, m->n_big + single, m->max_teams});
+    const int slots = nsm * per_sm;
+    p.team = mg::kTeamMin;
+    while (p.team < mg::kTeamMax && 2 * p.team * m->n_big <= slots) p.team *= 2;
+    const int single = (m->n - m->n_big + p.team - 1) / p.team;
+    const int teams = std::min({slots / p.team, m->n_big + single, m->max_teams});
     if (teams < 1) return set_error(XBFS_ERR_INTERNAL, "multi-graph kernel cannot be resident");
-    XBFS_CUDA_TRY(cudaLaunchCooperativeKernel(kfn, dim3(teams * mg::kTeam), dim3(block), args, smem, s));
+    XBFS_CUDA_TRY(cudaLaunchCooperativeKernel(kfn, dim3(teams * p.team), dim3(block), args, smem, s));
   } else {
     XBFS_CUDA_TRY(cudaLaunchKernel(kfn, dim3(std::min(nsm * per_sm, m->n)), dim3(block), args, smem, s));
   }
@@ -661,7 +671,7 @@ xbfs_status xbfs_multi_create(xbfs_graph* const* graphs, int32_t n, int32_t devi
   if (m->n_big > 0) {
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-    m->max_teams = std::max(1, nsm * 2 / mg::kTeam);  // shared memory admits two CTAs per SM
+    m->max_teams = std::max(1, nsm * 2 / mg::kTeamMin);  // shared memory admits two CTAs per SM
     m->team_words = (big_v + 31) / 32;
     m->heavy_cap = big_long + 1;
     if ((st = m->bits.ensure((size_t)m->max_teams * 4 * (size_t)m->team_words * 4)) ||
