@@ -73,35 +73,63 @@ struct Params {
   Ctl* ctl;
 };
 
+// What a round's CTA keeps in shared memory.
+struct Tick {
+  int* out[kSlots];                 // the slots' tables, which change between rounds only
+  long long join[kSlots];
+  unsigned long long msum[kSlots];  // per slot: degrees of the vertices gained at this tick
+  unsigned long long act;           // slots that gained a vertex
+  int mine;                         // entries of wu that this CTA expanded at the last tick (-1: not all kept)
+  int next_s;
+  long long wbeg[kBlock + 1];
+  unsigned web[kBlock + 1];
+  int wu[kBlock + 1];
+};
+
 // Claim step of one edge (u, v) at tick t (see sv_tick), u offering the
 // slot mask fu; returns whether this thread queues v for tick t+1, with v's
-// degree and CSR offset.
-__device__ __forceinline__ bool sv_claim_m(const Params& p, long long t, unsigned long long fu,
-                                           unsigned long long* Fn, int v, long long& deg, long long& b0,
-                                           unsigned long long& act, unsigned long long* s_msum) {
-  const unsigned long long m = fu & ~ld_cg_u64(p.vis + v);
+// degree and CSR offset; `gained` are the slots that v got here. SPEC: the
+// atomic is issued without a look at the visited word before (small queues,
+// where the extra read would only lengthen the tick). The CSR offsets are read
+// beside the atomic.
+template <bool SPEC>
+__device__ __forceinline__ bool sv_claim(const Params& p, const Tick& k, long long t, unsigned long long fu,
+                                         unsigned long long* Fn, int v, long long& deg, long long& b0,
+                                         unsigned long long& gained) {
+  gained = 0ull;
+  const unsigned long long m = SPEC ? fu : fu & ~ld_cg_u64(p.vis + v);
   if (!m) return false;
-  const unsigned long long gained = m & ~atomicOr(p.vis + v, m);
-  if (!gained) return false;
-  b0 = ld_nc_i64(p.beg + v);
-  deg = ld_nc_i64(p.beg + v + 1) - b0;
+  const long long x0 = ld_nc_i64(p.beg + v), x1 = ld_nc_i64(p.beg + v + 1);
+  const unsigned long long g = m & ~atomicOr(p.vis + v, m);
+  if (!g) return false;
+  b0 = x0;
+  deg = x1 - x0;
+  gained = g;
   // a vertex without edges is never expanded: it gets levels, no frontier bits
-  const unsigned long long prev = deg > 0 ? atomicOr(Fn + v, gained) : ~0ull;
-  act |= gained;
-  for (unsigned long long bits = gained; bits; bits &= bits - 1) {
+  const unsigned long long prev = deg > 0 ? atomicOr(Fn + v, g) : ~0ull;
+  for (unsigned long long bits = g; bits; bits &= bits - 1) {
     const int sl = __ffsll((long long)bits) - 1;
-    int* o = p.out[sl];
-    if (o) o[v] = (int)(t + 1 - p.join[sl]);
-    if (deg) atomicAdd(&s_msum[sl], (unsigned long long)deg);
+    int* o = k.out[sl];
+    if (o) o[v] = (int)(t + 1 - k.join[sl]);
   }
-  return prev == 0 && deg > 0;
+  return prev == 0;
 }
 
-// The same with u's whole frontier mask.
-__device__ __forceinline__ bool sv_claim(const Params& p, long long t, const unsigned long long* Fc,
-                                         unsigned long long* Fn, int u, int v, long long& deg, long long& b0,
-                                         unsigned long long& act, unsigned long long* s_msum) {
-  return sv_claim_m(p, t, ld_cg_u64(Fc + u), Fn, v, deg, b0, act, s_msum);
+// Books what the lanes of a full warp gained: degrees per slot (summed over
+// the warp first: a slot's lanes would otherwise meet on one 64-bit word of
+// shared memory) and the slots.
+__device__ __forceinline__ void sv_account(Tick& k, unsigned long long gained, long long deg) {
+  if (!__any_sync(0xffffffffu, gained != 0ull)) return;
+  const int lane = threadIdx.x & 31;
+  unsigned long long all = __reduce_or_sync(0xffffffffu, (unsigned)gained) |
+                           ((unsigned long long)__reduce_or_sync(0xffffffffu, (unsigned)(gained >> 32)) << 32);
+  if (lane == 0) atomicOr(&k.act, all);
+  for (; all; all &= all - 1) {
+    const int sl = __ffsll((long long)all) - 1;
+    // distinct vertices: their degrees sum to at most E < 2^32
+    const unsigned d = __reduce_add_sync(0xffffffffu, (gained >> sl) & 1ull ? (unsigned)deg : 0u);
+    if (lane == 0 && d) atomicAdd(&k.msum[sl], (unsigned long long)d);
+  }
 }
 
 // Warp-aggregated append of the lanes with `have` to queue qn (full warp).
@@ -129,31 +157,31 @@ __device__ __forceinline__ void sv_enqueue(const Params& p, int qn, bool have, i
 // frontier mask, and the thread whose OR found v's next mask empty queues v
 // for tick t+1 (so v is queued once). Edge-balanced: part takes an equal
 // share of the queue's edges.
-__device__ void sv_tick(const Params& p, long long t, unsigned nparts, unsigned part,
-                        unsigned long long* s_msum, unsigned long long* s_act) {
-  __shared__ long long wbeg[kBlock + 1];
-  __shared__ unsigned web[kBlock + 1];
-  __shared__ int wu[kBlock + 1];
-  __shared__ int next_s;
+// pk: the queue's packed counter.
+__device__ void sv_tick(const Params& p, Tick& k, long long t, unsigned nparts, unsigned part,
+                        unsigned long long pk) {
+  long long* wbeg = k.wbeg;
+  unsigned* web = k.web;
+  int* wu = k.wu;
   const int lane = threadIdx.x & 31;
   const int qs = (int)(t % 4), qn = (int)((t + 1) % 4);
-  const unsigned long long pk = ld_cg_u64(&p.ctl->q[qs]);
   const unsigned cnt = (unsigned)(pk & kCountMask);
   const unsigned long long M = pk >> 31;
   const unsigned long long G = nparts;
   const unsigned long long lo = M * part / G, hi = M * (part + 1) / G;
+  const bool small = (unsigned long long)cnt <= 32ull * G && M <= 32ull * cnt;
+  const unsigned i0 = (unsigned)((unsigned long long)cnt * part / G);
+  const unsigned i1 = (unsigned)((unsigned long long)cnt * (part + 1) / G);
+  if (threadIdx.x == 0) k.mine = small ? (int)(i1 - i0) : -1;
   if (cnt == 0) return;
   const int* ids = p.qids[qs];
   const unsigned* eb = p.qeb[qs];
   const long long* bgs = p.qbg[qs];
   const unsigned long long* Fc = p.F[t % 3];
   unsigned long long* Fn = p.F[(t + 1) % 3];
-  unsigned long long act = 0;
-  if ((unsigned long long)cnt <= 32ull * G && M <= 32ull * cnt) {
+  if (small) {
     // small queue of low-degree vertices: each part takes an equal share of
     // the entries (at most 32), so no part searches the queue for its start
-    const unsigned i0 = (unsigned)((unsigned long long)cnt * part / G);
-    const unsigned i1 = (unsigned)((unsigned long long)cnt * (part + 1) / G);
     if (i0 >= i1) return;
     const int n = (int)(i1 - i0);
     const unsigned base = eb[i0];
@@ -167,9 +195,11 @@ __device__ void sv_tick(const Params& p, long long t, unsigned nparts, unsigned 
     __syncthreads();
     for (unsigned long long e0 = 0; e0 < T; e0 += kBlock) {
       const unsigned long long e = e0 + threadIdx.x;
+      if ((e & ~31ull) >= T) break;  // whole warps
       bool first = false;
       int v = 0;
       long long deg = 0, b0 = 0;
+      unsigned long long gained = 0ull;
       if (e < T) {
         int a = 0, c = n;
         while (c - a > 1) {
@@ -177,9 +207,10 @@ __device__ void sv_tick(const Params& p, long long t, unsigned nparts, unsigned 
           if ((unsigned long long)web[mid] <= e) a = mid; else c = mid;
         }
         v = ld_stream_i32(p.csr + wbeg[a] + (long long)(e - web[a]));
-        first = sv_claim(p, t, Fc, Fn, wu[a], v, deg, b0, act, s_msum);
+        first = sv_claim<true>(p, k, t, ld_cg_u64(Fc + wu[a]), Fn, v, deg, b0, gained);
       }
       sv_enqueue(p, qn, first, v, deg, b0);
+      sv_account(k, gained, deg);
     }
   } else if (lo < hi) {
   if (threadIdx.x < 32) {
@@ -196,10 +227,10 @@ __device__ void sv_tick(const Params& p, long long t, unsigned nparts, unsigned 
     }
     const unsigned idx = a + lane;
     const unsigned m = __ballot_sync(0xffffffffu, idx < b && (unsigned long long)eb[idx] <= lo);
-    if (lane == 0) next_s = (int)(a + 31 - __clz(m));
+    if (lane == 0) k.next_s = (int)(a + 31 - __clz(m));
   }
   __syncthreads();
-  unsigned s = (unsigned)next_s;
+  unsigned s = (unsigned)k.next_s;
   for (unsigned long long r = lo; r < hi; r += kBlock) {
     const unsigned long long rhi = (r + kBlock < hi) ? r + kBlock : hi;
     for (int i = threadIdx.x; i <= kBlock; i += kBlock) {
@@ -220,6 +251,7 @@ __device__ void sv_tick(const Params& p, long long t, unsigned nparts, unsigned 
     bool first = false;
     int v = 0;
     long long deg = 0, b0 = 0;
+    unsigned long long gained = 0ull;
     if (e < rhi) {
       int a = 0, c = kBlock + 1;
       while (c - a > 1) {
@@ -227,32 +259,30 @@ __device__ void sv_tick(const Params& p, long long t, unsigned nparts, unsigned 
         if ((unsigned long long)web[mid] <= e) a = mid; else c = mid;
       }
       v = ld_stream_i32(p.csr + wbeg[a] + (long long)(e - web[a]));
-      first = sv_claim(p, t, Fc, Fn, wu[a], v, deg, b0, act, s_msum);
+      first = sv_claim<false>(p, k, t, ld_cg_u64(Fc + wu[a]), Fn, v, deg, b0, gained);
     }
     sv_enqueue(p, qn, first, v, deg, b0);
+    sv_account(k, gained, deg);
     if (threadIdx.x == 0 && rhi < hi) {
       int a = 0, c = kBlock + 1;
       while (c - a > 1) {
         const int mid = (a + c) >> 1;
         if ((unsigned long long)web[mid] <= rhi) a = mid; else c = mid;
       }
-      next_s = (int)(s + a);
+      k.next_s = (int)(s + a);
     }
     __syncthreads();
-    s = (unsigned)next_s;
+    s = (unsigned)k.next_s;
   }
   }
-  act = __reduce_or_sync(0xffffffffu, (unsigned)act) |
-        ((unsigned long long)__reduce_or_sync(0xffffffffu, (unsigned)(act >> 32)) << 32);
-  if (lane == 0 && act) atomicOr(s_act, act);
 }
 
 // Top-down part of a mixed tick t: the queue entries whose frontier mask
 // holds bits of `mask` (the slots not advanced bottom-up at this tick) are
 // compacted per block (each block takes an equal share of the entries) and
 // their edges expanded across the block for those bits only.
-__device__ void sv_tick_td_part(const Params& p, long long t, unsigned long long mask, unsigned nparts,
-                                unsigned part, unsigned long long* s_msum, unsigned long long& act) {
+__device__ void sv_tick_td_part(const Params& p, Tick& k, long long t, unsigned long long mask, unsigned nparts,
+                                unsigned part) {
   __shared__ int cu[kBlock];
   __shared__ unsigned long long cm[kBlock];
   __shared__ long long cb[kBlock];
@@ -282,11 +312,11 @@ __device__ void sv_tick_td_part(const Params& p, long long t, unsigned long long
     const unsigned long long x =
         block_exclusive_scan<kBlock, unsigned long long>(fu ? (d << 16) | 1ull : 0ull, s_scan, &tot);
     if (fu) {
-      const int k = (int)(x & 0xffffull);
-      cu[k] = u;
-      cm[k] = fu;
-      cb[k] = b0;
-      ce[k] = x >> 16;
+      const int at = (int)(x & 0xffffull);
+      cu[at] = u;
+      cm[at] = fu;
+      cb[at] = b0;
+      ce[at] = x >> 16;
     }
     __syncthreads();
     const int n = (int)(tot & 0xffffull);
@@ -296,6 +326,7 @@ __device__ void sv_tick_td_part(const Params& p, long long t, unsigned long long
       bool first = false;
       int v = 0;
       long long deg = 0, vb0 = 0;
+      unsigned long long gained = 0ull;
       if (e < T) {
         int a = 0, c = n;
         while (c - a > 1) {
@@ -303,9 +334,10 @@ __device__ void sv_tick_td_part(const Params& p, long long t, unsigned long long
           if (ce[mid] <= e) a = mid; else c = mid;
         }
         v = ld_stream_i32(p.csr + cb[a] + (long long)(e - ce[a]));
-        first = sv_claim_m(p, t, cm[a], Fn, v, deg, vb0, act, s_msum);
+        first = sv_claim<false>(p, k, t, cm[a], Fn, v, deg, vb0, gained);
       }
       sv_enqueue(p, qn, first, v, deg, vb0);
+      sv_account(k, gained, deg);
     }
     __syncthreads();
   }
@@ -320,20 +352,20 @@ __device__ void sv_tick_td_part(const Params& p, long long t, unsigned long long
 // parts claim disjoint bits, so visited and next-frontier words take atomic
 // ORs and the OR that finds v's next mask empty queues v. Blocks take
 // contiguous vertex ranges.
-__device__ void sv_tick_bu(const Params& p, long long t, unsigned long long bu, unsigned long long td,
-                           unsigned nparts, unsigned part, unsigned long long* s_msum, unsigned long long* s_act) {
-  const int lane = threadIdx.x & 31;
+__device__ void sv_tick_bu(const Params& p, Tick& k, long long t, unsigned long long bu, unsigned long long td,
+                           unsigned nparts, unsigned part) {
   const int qn = (int)((t + 1) % 4);
   const unsigned long long* Fc = p.F[t % 3];
   unsigned long long* Fn = p.F[(t + 1) % 3];
-  unsigned long long act = 0;
-  if (td) sv_tick_td_part(p, t, td, nparts, part, s_msum, act);
+  if (threadIdx.x == 0) k.mine = -1;
+  if (td) sv_tick_td_part(p, k, t, td, nparts, part);
   const long long per = (p.V + nparts - 1) / nparts;
   const long long v0 = per * part, v1 = (v0 + per < p.V) ? v0 + per : p.V;
   for (long long base = v0; base < v1; base += blockDim.x) {
     const long long v = base + threadIdx.x;
     bool have = false;
     long long deg = 0, vb0 = 0;
+    unsigned long long gained = 0ull;
     if (v < v1) {
       const unsigned long long vv = ld_cg_u64(p.vis + v);
       const unsigned long long needed = bu & ~vv;
@@ -345,10 +377,10 @@ __device__ void sv_tick_bu(const Params& p, long long t, unsigned long long bu, 
         for (long long e = b0; e < b1 && got != needed; e += 4) {
           int u[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) u[k] = (e + k < b1) ? ld_stream_i32(p.csr + e + k) : -1;
+          for (int j = 0; j < 4; ++j) u[j] = (e + j < b1) ? ld_stream_i32(p.csr + e + j) : -1;
           unsigned long long f[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) f[k] = (u[k] >= 0) ? ld_cg_u64(Fc + u[k]) : 0ull;
+          for (int j = 0; j < 4; ++j) f[j] = (u[j] >= 0) ? ld_cg_u64(Fc + u[j]) : 0ull;
           got |= (f[0] | f[1] | f[2] | f[3]) & needed;
         }
         if (got) {
@@ -356,21 +388,18 @@ __device__ void sv_tick_bu(const Params& p, long long t, unsigned long long bu, 
           vb0 = b0;
           atomicOr(p.vis + v, got);
           have = atomicOr(Fn + v, got) == 0ull;
-          act |= got;
+          gained = got;
           for (unsigned long long bits = got; bits; bits &= bits - 1) {
             const int sl = __ffsll((long long)bits) - 1;
-            int* o = p.out[sl];
-            if (o) o[v] = (int)(t + 1 - p.join[sl]);
-            atomicAdd(&s_msum[sl], (unsigned long long)deg);
+            int* o = k.out[sl];
+            if (o) o[v] = (int)(t + 1 - k.join[sl]);
           }
         }
       }
     }
     sv_enqueue(p, qn, have, (int)v, deg, vb0);
+    sv_account(k, gained, deg);
   }
-  act = __reduce_or_sync(0xffffffffu, (unsigned)act) |
-        ((unsigned long long)__reduce_or_sync(0xffffffffu, (unsigned)(act >> 32)) << 32);
-  if (lane == 0 && act) atomicOr(s_act, act);
 }
 
 // Clears the frontier masks of tick t (the vertices of queue t).
@@ -397,15 +426,22 @@ constexpr long long kBuRatio = 8;
 
 __global__ void __launch_bounds__(kBlock) k_sv_round(Params p, long long t0, int k, unsigned long long timeout_ns,
                                                      unsigned long long running) {
-  __shared__ unsigned long long s_msum[kSlots];
-  __shared__ unsigned long long s_act;
+  __shared__ Tick tk;
   __shared__ unsigned s_bu[2], s_live[2];
   const unsigned G = gridDim.x, b = blockIdx.x;
   uint32_t epoch = 0;
+  if (threadIdx.x < kSlots) {
+    tk.out[threadIdx.x] = p.out[threadIdx.x];
+    tk.join[threadIdx.x] = p.join[threadIdx.x];
+  }
+  if (threadIdx.x == 0) tk.mine = -1;
+  __syncthreads();
   for (int i = 0; i < k; ++i) {
     const long long t = t0 + i;
+    // this tick's queue length, read beside the slots' frontier edges
+    const unsigned long long pk = ld_cg_u64(&p.ctl->q[t % 4]);
     if (threadIdx.x < kSlots) {
-      s_msum[threadIdx.x] = 0;
+      tk.msum[threadIdx.x] = 0;
       const unsigned long long f = ld_cg_u64(&p.ctl->fe[t % 4][threadIdx.x]);
       const bool big = p.allow_bu && ((running >> threadIdx.x) & 1ull) && (long long)f * kBuRatio > p.E;
       const unsigned bb = __ballot_sync(0xffffffffu, big), lb = __ballot_sync(0xffffffffu, f != 0);
@@ -415,26 +451,33 @@ __global__ void __launch_bounds__(kBlock) k_sv_round(Params p, long long t0, int
       }
       if (b == 0) p.ctl->fe[(t + 2) % 4][threadIdx.x] = 0ull;
     }
-    if (threadIdx.x == 0) s_act = 0;
+    if (threadIdx.x == 0) tk.act = 0;
     if (b == 0 && threadIdx.x == 0) {
       p.ctl->q[(t + 2) % 4] = 0ull;
       // the first tick's activity word is zeroed by the host before the round
       if (i + 1 < k) p.ctl->active[(t + 1) % kRing] = 0ull;
     }
+    // frontier t-1's masks: the entries this CTA expanded itself, where it
+    // still has them, else its part of the queue
+    const int mine = tk.mine;
+    if (mine >= 0) {
+      if ((int)threadIdx.x < mine) p.F[(t + 2) % 3][tk.wu[threadIdx.x]] = 0ull;
+    } else if (t > 0) {
+      sv_retire(p, t - 1, G, b);
+    }
     __syncthreads();
-    if (t > 0) sv_retire(p, t - 1, G, b);
     const unsigned long long bu = s_bu[0] | ((unsigned long long)s_bu[1] << 32);
     const unsigned long long live = s_live[0] | ((unsigned long long)s_live[1] << 32);
     if (bu)
-      sv_tick_bu(p, t, bu, running & live & ~bu, G, b, s_msum, &s_act);
+      sv_tick_bu(p, tk, t, bu, running & live & ~bu, G, b);
     else
-      sv_tick(p, t, G, b, s_msum, &s_act);
+      sv_tick(p, tk, t, G, b, pk);
     __syncthreads();
-    if (threadIdx.x < kSlots && s_msum[threadIdx.x]) {
-      atomicAdd(&p.ctl->msum[threadIdx.x], s_msum[threadIdx.x]);
-      atomicAdd(&p.ctl->fe[(t + 1) % 4][threadIdx.x], s_msum[threadIdx.x]);
+    if (threadIdx.x < kSlots && tk.msum[threadIdx.x]) {
+      atomicAdd(&p.ctl->msum[threadIdx.x], tk.msum[threadIdx.x]);
+      atomicAdd(&p.ctl->fe[(t + 1) % 4][threadIdx.x], tk.msum[threadIdx.x]);
     }
-    if (threadIdx.x == 0 && s_act) atomicOr(&p.ctl->active[t % kRing], s_act);
+    if (threadIdx.x == 0 && tk.act) atomicOr(&p.ctl->active[t % kRing], tk.act);
     if (!grid_sync(&p.ctl->bar, G, epoch, timeout_ns)) return;
   }
 }
@@ -812,8 +855,11 @@ static xbfs_status engine_step(Server* srv, bool oom_is_error, bool* active, boo
     int grid = b.grid;
     if (b.tick > 0 && b.depth_est >= kDeepGraph) {
       const unsigned long long pk = hctl[gi].q[b.tick % 4];
-      const unsigned long long work = std::max<unsigned long long>(pk >> 31, pk & sv::kCountMask);
-      const unsigned long long want = (work * 4 + sv::kBlock * 2 - 1) / (sv::kBlock * 2);
+      const unsigned long long cnt = pk & sv::kCountMask, work = std::max<unsigned long long>(pk >> 31, cnt);
+      // and room for its entries to double with at most 32 of them per block
+      // (sv_tick's small queues: no search, one round of edges)
+      const unsigned long long want =
+          std::max<unsigned long long>((work * 4 + sv::kBlock * 2 - 1) / (sv::kBlock * 2), (cnt + 15) / 16);
       grid = (int)std::min<unsigned long long>((unsigned long long)b.grid, std::max<unsigned long long>(8, want));
     }
     grid = std::min(grid, std::max(8, b.max_coop / std::max(1, with_work)));
