@@ -379,3 +379,33 @@ def test_degree_sorted_adjacency_keeps_levels():
     g.sort_adjacency("id")
     assert np.array_equal(g.download()[1], csr)
     g.free()
+
+
+@pytest.mark.parametrize("forced", [None, ["td_queue"], ["td_queue", "td_scan"], ["td_queue", "bu", "td_queue"]])
+def test_small_queues_over_all_bins(forced):
+    """Levels whose queue has few entries in all three degree bins (one pass
+    over the concatenated bins), with winners on both sides of what one warp
+    per bin flushes, and Erdos-Renyi levels around 32 entries per CTA."""
+    rng = np.random.default_rng(3)
+    degs = [3, 32, 33, 200, 256, 257, 300, 3000, 1, 2] + [5] * 90 + [40] * 130 + [300] * 20
+    pairs, V = [], 1 + len(degs)
+    for i, d in enumerate(degs):
+        pairs.append((0, 1 + i))
+        pairs += [(1 + i, V + k) for k in range(d - 1)]
+        V += d - 1
+    pairs += [(int(a), int(b)) for a, b in rng.integers(1, V, size=(3000, 2))]
+    e = np.array(pairs, dtype=np.int64)
+    e = np.concatenate([e, e[:, ::-1]])
+    e = e[np.lexsort((e[:, 1], e[:, 0]))]
+    beg = np.concatenate([[0], np.cumsum(np.bincount(e[:, 0], minlength=V))]).astype(np.int64)
+    sets = [(beg, e[:, 1].astype(np.int32), [0, 1, V - 1, 8]), gen_er_host(300000, 8.0, 4) + ([5, 77, 4711],)]
+    kw = {"policy": "forced", "forced": forced} if forced else {}
+    for b, c, srcs in sets:
+        g = Graph.from_csr(b, c)
+        for grid_dim in (0, 3):
+            for s in srcs:
+                r = g.bfs(int(s), want_parents=True, grid_dim=grid_dim, **kw)
+                ref = oracle.bfs_queue(b, c, int(s))
+                assert np.array_equal(r.levels, ref)
+                assert oracle.check_tree(b, c, int(s), r.levels, r.parents) == 0
+                assert r.reached == int((ref >= 0).sum())

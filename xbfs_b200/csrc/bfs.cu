@@ -145,6 +145,11 @@ constexpr int kRoundsNoStage = 4;   // edge-balanced rounds with bitmap output: 
 constexpr int kTdIlp = XBFS_TD_ILP; // edges per thread in flight in the barrier-free top-down loops
 constexpr int kCap = 1024;          // staging capacity, small and medium bins
 constexpr int kCapL = 256;          // staging capacity, large bin
+// Edges per CTA up to which one warp expands a CTA's share alone: its rounds of
+// 32 edges take 2 us each, a block's one round 9 (an Erdos-Renyi level of 9,543
+// vertices and 85,624 edges, 32 entries per CTA: 33 us by warps, 14 by blocks).
+constexpr int kTinyEdges = 64;
+constexpr int kFlushWarp = 128;     // up to this many staged entries per bin are flushed by one warp each
 constexpr int kFlushAt = kCap - kTE;  // a round adds at most kTE winners: flush before each
 constexpr int kFlushAtL = kCapL / 2;  // large-bin overflow goes straight to the global queue
 static_assert(kFlushAt >= 0, "a gather round must fit the staging area");
@@ -347,6 +352,7 @@ struct __align__(16) Smem {
   float few_margin;
   int few_dec;
   int fitted;                   // levels in a row that would have fitted a run
+  long long fit_m;              // the last level's degree sum
   unsigned waiting;             // thread 0: CTAs that have waited for runs' ends so far
   float mlp_w[1472];            // the learned switch's weights and bound (XBFS_POLICY_MLP); must stay last
 };
@@ -617,6 +623,42 @@ __device__ __forceinline__ void stage(Smem& sm, const QOut& q, int bin, int v, l
 // Block-wide flush of all staged winners (call from all threads, uniform).
 __device__ void flush(Smem& sm, const QOut& q) {
   __syncthreads();
+  if (sm.cnt[0] <= kFlushWarp && sm.cnt[1] <= kFlushWarp && sm.cnt[2] <= kFlushWarp) {
+    // few winners: one warp per bin, the bins side by side
+    const int bin = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n = bin < 3 ? sm.cnt[bin] : 0;
+    if (n > 0) {
+      const int* ids = bin < 2 ? sm.st_id[bin] : sm.stl_id;
+      const int* degs = bin < 2 ? sm.st_deg[bin] : sm.stl_deg;
+      const long long* bgs = bin < 2 ? sm.st_bg[bin] : sm.stl_bg;
+      long long d[kFlushWarp / 32], loc = 0;
+#pragma unroll
+      for (int k = 0; k < kFlushWarp / 32; ++k) {
+        d[k] = lane * (kFlushWarp / 32) + k < n ? degs[lane * (kFlushWarp / 32) + k] : 0;
+        loc += d[k];
+      }
+      const long long inc = warp_inclusive_scan(loc);
+      unsigned long long old = 0;
+      if (lane == 31) old = atomicAdd(&q.ctr[bin], ((unsigned long long)inc << 31) | (unsigned long long)n);
+      old = __shfl_sync(0xffffffffu, old, 31);
+      const unsigned long long bs = old & kCountMask;
+      long long run = (long long)(old >> 31) + inc - loc;
+#pragma unroll
+      for (int k = 0; k < kFlushWarp / 32; ++k) {
+        const int i = lane * (kFlushWarp / 32) + k;
+        if (i < n) {
+          q.b[bin].ids[bs + i] = ids[i];
+          q.b[bin].eb[bs + i] = (unsigned)run;
+          q.b[bin].bg[bs + i] = bgs[i];
+          run += d[k];
+        }
+      }
+      __syncwarp();
+      if (lane == 0) sm.cnt[bin] = 0;
+    }
+    __syncthreads();
+    return;
+  }
   for (int bin = 0; bin < 3; ++bin) {
     const int cap = bin < 2 ? kCap : kCapL;
     int n = sm.cnt[bin];
@@ -940,6 +982,48 @@ __device__ void gather_bin_warp(const Params& p, Acc& acc, const QOut& q, const 
       s += 32;
     }
   }
+}
+
+// The whole queue of a level with few entries (at most kWin over the three
+// bins) and at most one round of edges per CTA: every CTA loads all entries and
+// takes its share of the concatenated edge space (large bin first), so the
+// level is one chain of reads instead of one per bin with a search each. The
+// first levels of a power-law graph, a few vertices of degrees in every bin, take
+// this path (level 1 of R-MAT scale 16: 14 -> 9 us).
+template <bool PAR>
+__device__ void gather_all(const Params& p, Smem& sm, const QOut& q, Acc& acc, const QBin* in, int L, bool enq,
+                           uint32_t* fbn, bool qside) {
+  const unsigned c2 = (unsigned)(sm.bins[2] & kCountMask), c1 = (unsigned)(sm.bins[1] & kCountMask);
+  const unsigned n = c2 + c1 + (unsigned)(sm.bins[0] & kCountMask);
+  const unsigned m2 = (unsigned)(sm.bins[2] >> 31), m1 = (unsigned)(sm.bins[1] >> 31);
+  const unsigned T = m2 + m1 + (unsigned)(sm.bins[0] >> 31);
+  const unsigned lo = (unsigned)((unsigned long long)T * blockIdx.x / gridDim.x);
+  const unsigned hi = (unsigned)((unsigned long long)T * (blockIdx.x + 1) / gridDim.x);
+  if (lo >= hi) return;
+  const bool spec = sm.spec != 0;
+  for (unsigned i = threadIdx.x; i < n; i += kBlock) {
+    const int b = i < c2 ? 2 : (i < c2 + c1 ? 1 : 0);
+    const unsigned slot = b == 2 ? i : (b == 1 ? i - c2 : i - c2 - c1);
+    sm.web[i] = in[b].eb[slot] + (b == 2 ? 0u : (b == 1 ? m2 : m2 + m1));
+    sm.wu[i] = in[b].ids[slot];
+    sm.wbeg[i] = in[b].bg[slot];
+  }
+  __syncthreads();
+  int v[kK], u[kK];
+#pragma unroll
+  for (int k = 0; k < kK; ++k) {
+    const unsigned e = lo + threadIdx.x + (unsigned)k * kBlock;
+    v[k] = -1;
+    u[k] = 0;
+    if (e < hi) {
+      const int a = smem_owner(sm.web, (int)n, e);
+      v[k] = ld_stream_i32(p.csr + sm.wbeg[a] + (long long)(e - sm.web[a]));
+      u[k] = sm.wu[a];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kK; ++k)
+    if (v[k] >= 0) claim_td<PAR>(p, sm, q, acc, v[k], u[k], L, enq, fbn, spec, qside);
 }
 
 // Edge-balanced expansion of one bin of the current frontier queue (medium
@@ -2321,7 +2405,7 @@ __device__ __forceinline__ int decide_learned(Smem& sm, long long L, long long n
 // small_max edges or more edges than fit was found; what is left in shared
 // memory then becomes the binned queue again. Entering and leaving costs about
 // what a level of the whole grid does, so a run starts after kFewAfter levels
-// that would have fitted (R-MAT and Erdos-Renyi graphs have up to five).
+// that would have fitted and grew by at most half.
 struct FewSmem {
   unsigned pos[2][kFewEdges];  // CSR position of every frontier edge, by level parity
   int u[2][kFewEdges];         // the frontier vertex it belongs to
@@ -2547,23 +2631,24 @@ __device__ __noinline__ void few_aside(const Params& p, Smem& sm, unsigned L0) {
   }
 }
 
-// Learned switch: decision for a level outside the box (full warp).
-// t: the level before the one to decide.
+// Learned switch: decision for a level outside the box (full warp), by the
+// network. t: the level before the one to decide.
 __device__ __noinline__ int few_decide_learned(const Params& p, Smem& sm, const FewStat& t, unsigned n, unsigned m) {
   const int lane = threadIdx.x & 31;
-  int s = XBFS_TD_QUEUE;
-  if (lane == 0) {
-    sm.ls.ps.n_prev = t.n;
-    s = decide_learned(sm, (long long)t.level + 1, n, m, max(p.n_ni - (long long)t.vn - n, 0ll),
-                       max(p.E - (long long)t.vm - m, 0ll));
-  }
-  s = __shfl_sync(0xffffffffu, s, 0);
-  if (s == -2) {
-    s = mlp_decide(sm.mlp_w, sm.mlp_raw, sm.mlp_act, lane, sm.mlp_cache_raw, &sm.mlp_cache_dec, &sm.mlp_cache_margin);
-    s = __shfl_sync(0xffffffffu, s, 0);
-  }
+  const unsigned n_ni = (unsigned)p.n_ni, E = (unsigned)p.E, vn = t.vn + n, vm = t.vm + m;
+  float v = 0.f;  // lane 5: the strategy of the level before, XBFS_TD_QUEUE
+  if (lane == 0) v = (float)n;
+  if (lane == 1) v = (float)m;
+  if (lane == 2) v = vn < n_ni ? (float)(n_ni - vn) : 0.f;
+  if (lane == 3) v = vm < E ? (float)(E - vm) : 0.f;
+  if (lane == 4) v = (float)(t.level + 1);
+  if (lane == 6) v = (float)t.n;
+  if (lane == 7) v = (float)m / (float)n;
+  if (lane < 8) sm.mlp_raw[lane] = v;
   __syncwarp();
-  return s;
+  const int s = mlp_decide(sm.mlp_w, sm.mlp_raw, sm.mlp_act, lane, sm.mlp_cache_raw, &sm.mlp_cache_dec,
+                           &sm.mlp_cache_margin);
+  return __shfl_sync(0xffffffffu, s, 0);
 }
 
 // Counts of one level across the run's CTAs (full warp): each writes one word
@@ -2681,10 +2766,17 @@ __device__ __noinline__ bool small_levels(const Params& p, Smem& sm, long long L
       for (;;) {
         const int par = (int)(L & 1);
         if (LEARNED && threadIdx.x < 32) {
-          // the box as it is now, while the others claim
+          // the box as it is now, while the others claim, as ranges of the
+          // next level's two counts: what it says of the visited sums, the
+          // level and the growth becomes part of n's and m's
           const unsigned made = sm.few_made;
           sure = sm.few_sure[made & 1];
-          if (sm.few_made != made) sure.n_lo = ~0u;  // being drawn anew
+          const float grown = (float)st.n + 1.f;
+          sure.n_lo = max(sure.n_lo, (unsigned)fmaxf(ceilf(sure.g_lo * grown - 1.f), 0.f));
+          sure.n_hi = min(min(sure.n_hi, (unsigned)fmaxf(sure.g_hi * grown - 1.f, 0.f)),
+                          max(sure.vn_hi, st.vn) - st.vn);
+          sure.m_hi = min(sure.m_hi, max(sure.vm_hi, st.vm) - st.vm);
+          if (sm.few_made != made || st.level + 1 > sure.level_hi) sure.n_lo = ~0u;  // being drawn anew, or left
         }
         if (threadIdx.x >= 32 && (e0 & ~31u) < m) {  // whole warps
           for (unsigned e = e0;;) {
@@ -2710,7 +2802,9 @@ __device__ __noinline__ bool small_levels(const Params& p, Smem& sm, long long L
             PolicyState next = ps;
             int s = XBFS_TD_QUEUE;
             if (LEARNED) {
-              if (!few_inside(sure, n_s, m_s, st.vn + n_s, st.vm + m_s, st.level + 1, st.n))
+              const float n_f = (float)n_s, m_f = (float)m_s;
+              if (!(n_s >= sure.n_lo && n_s <= sure.n_hi && m_s >= sure.m_lo && m_s <= sure.m_hi &&
+                    m_f >= sure.d_lo * n_f && m_f <= sure.d_hi * n_f))
                 s = few_decide_learned(p, sm, st, n_s, m_s);
             } else {
               s = decide(p, next, (long long)st.level + 1, n_s, m_s, max(p.E - (long long)st.vm - m_s, 0ll));
@@ -2924,6 +3018,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(const __grid_constant__ Param
   if (threadIdx.x == 0) {
     sm.waiting = 0;
     sm.fitted = 0;
+    sm.fit_m = 0;
   }
   if (p.fresh) {
     init_traversal<PAR>(p);
@@ -2993,13 +3088,17 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(const __grid_constant__ Param
       sm.few = 0;
       if ((unsigned long long)m_f <= (unsigned long long)(kFew * kFewShare) && pn == 0 &&
           (sm.bins[0] & kCountMask) != 0 && ((sm.bins[1] | sm.bins[2]) & kCountMask) == 0) {
-        if (++sm.fitted > kFewAfter && p.small_max <= kFewEdges - kFewShare) {
+        // a frontier that grows by more than half a level outgrows a run at
+        // once (what a run hands back is not compared with what came before it)
+        sm.fitted = from_run || m_f <= sm.fit_m + sm.fit_m / 2 + 64 ? sm.fitted + 1 : 0;
+        if (sm.fitted > kFewAfter && p.small_max <= kFewEdges - kFewShare) {
           const unsigned M = (unsigned)(sm.bins[0] >> 31), N = min((unsigned)kFew, gridDim.x);
           if (M <= N * kFewShare) sm.few = M <= (unsigned)kSoloIn ? 1 : (int)N;
         }
       } else {
         sm.fitted = 0;
       }
+      sm.fit_m = m_f;
       int s = -1;
       if (n_f > 0) {
         ls.vis_n += n_f;
@@ -3119,19 +3218,26 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(const __grid_constant__ Param
       QOut qo;
       for (int b2 = 0; b2 < 3; ++b2) qo.b[b2] = p.q[par ^ 1][b2];
       qo.ctr = F1->bin;
-      // a CTA whose whole share is at most 32 small-bin entries takes the
-      // warp-only path (no staging, no block reductions)
+      // a CTA whose whole share is at most 32 small-bin entries and about
+      // kTinyEdges edges takes the warp-only path (no staging, no block
+      // reductions)
       const unsigned long long pk0 = sm.bins[0];
       const unsigned cnt0 = (unsigned)(pk0 & kCountMask);
       const unsigned i0 = (unsigned)((unsigned long long)cnt0 * blockIdx.x / nb);
       const unsigned i1 = (unsigned)((unsigned long long)cnt0 * (blockIdx.x + 1) / nb);
-      const bool tiny = q_valid && (sm.bins[1] & kCountMask) == 0 && (sm.bins[2] & kCountMask) == 0 && i1 - i0 <= 32;
+      const bool tiny = q_valid && (sm.bins[1] & kCountMask) == 0 && (sm.bins[2] & kCountMask) == 0 && i1 - i0 <= 32 &&
+                        (pk0 >> 31) <= (unsigned long long)nb * kTinyEdges;
       if (tiny) {
         if (threadIdx.x < 32 && i1 > i0)
           gather_entries_warp<PAR>(p, qo, p.q[par][0], cnt0, pk0 >> 31, i0, i1, (int)L, enq, fbn, sm.spec != 0, P1,
                                    qside, mark == 2);
       } else {
-        if (q_valid) {
+        const unsigned long long entries =
+            cnt0 + (sm.bins[1] & kCountMask) + (sm.bins[2] & kCountMask);
+        const unsigned long long edges = (pk0 >> 31) + (sm.bins[1] >> 31) + (sm.bins[2] >> 31);
+        if (q_valid && !mark && entries <= (unsigned long long)kWin && edges <= (unsigned long long)nb * kTE) {
+          gather_all<PAR>(p, sm, qo, acc, p.q[par], (int)L, enq, fbn, qside);
+        } else if (q_valid) {
           for (int bin = 2; bin >= 1; --bin) {
             const unsigned long long pk = sm.bins[bin];
             gather_bin<PAR>(p, sm, qo, acc, p.q[par][bin], (unsigned)(pk & kCountMask), pk >> 31, (int)L, enq, fbn,
