@@ -50,6 +50,7 @@
 #include <limits.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <mutex>
 
@@ -3417,6 +3418,21 @@ static const void* bfs_kernel(bool parents, bool learned) {
   return parents ? (const void*)k_bfs<true, false> : (const void*)k_bfs<false, false>;
 }
 
+// CTAs of a launch: what the device holds at once, asked for once per device
+// and kernel (the query takes longer than the launch).
+static xbfs_status resident_grid(int device, bool parents, bool learned, const void* kfn, size_t smem, int* grid) {
+  static std::atomic<int> known[64][2][2];
+  std::atomic<int>* slot = device >= 0 && device < 64 ? &known[device][parents][learned] : nullptr;
+  if (slot && (*grid = slot->load(std::memory_order_relaxed)) > 0) return XBFS_OK;
+  int nsm = 0, per_sm = 0;
+  XBFS_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+  XBFS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kBlock, smem));
+  if (per_sm < 1) return set_error(XBFS_ERR_INTERNAL, "traversal kernel cannot be resident");
+  *grid = nsm * per_sm;
+  if (slot) slot->store(*grid, std::memory_order_relaxed);
+  return XBFS_OK;
+}
+
 // Fills the kernel parameters for one traversal of g with options o.
 static xbfs_status setup_params(Graph* g, const xbfs_opts& o, int* d_levels, int* d_parents, Params& p,
                                 const void** kfn_out, size_t* smem_out, int* grid_out) {
@@ -3471,11 +3487,8 @@ static xbfs_status setup_params(Graph* g, const xbfs_opts& o, int* d_levels, int
   // allocated for launches that use it (shared memory taken from L1)
   const size_t smem = sizeof(Smem) - (p.policy == XBFS_POLICY_MLP ? 0 : sizeof(((Smem*)0)->mlp_w));
   XBFS_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
-  int nsm = 0, per_sm = 0;
-  XBFS_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, g->device));
-  XBFS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kBlock, smem));
-  if (per_sm < 1) return set_error(XBFS_ERR_INTERNAL, "traversal kernel cannot be resident");
-  int grid = nsm * per_sm;
+  int grid = 0;
+  if (xbfs_status st = resident_grid(g->device, par_on, p.policy == XBFS_POLICY_MLP, kfn, smem, &grid)) return st;
   if (o.grid_dim > 0 && o.grid_dim < grid) grid = o.grid_dim;
   w.grid = grid;
   w.block = kBlock;
@@ -3578,8 +3591,16 @@ xbfs_status bfs_single(Graph* g, int32_t src, int32_t* levels, int32_t* parents,
   XBFS_CUDA_TRY(cudaEventRecord(w.evk0, s));
   XBFS_CUDA_TRY(cudaLaunchCooperativeKernel(kfn, dim3(grid), dim3(kBlock), args, smem, s));
   XBFS_CUDA_TRY(cudaEventRecord(w.ev1, s));
-  Ctl hctl;
-  XBFS_CUDA_TRY(cudaMemcpyAsync(&hctl, p.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
+  // results and the first levels' records come back together, into pinned
+  // memory; deeper traversals' other records are fetched once the depth is known
+  constexpr int kRecs = 64;
+  if ((st = w.result_pin.ensure(sizeof(Ctl) + sizeof(LevelRecDev) * kRecs))) return st;
+  const Ctl& hctl = *w.result_pin.as<Ctl>();
+  const LevelRecDev* hrec = reinterpret_cast<const LevelRecDev*>(w.result_pin.as<char>() + sizeof(Ctl));
+  const bool recs = o.trace || stats;
+  XBFS_CUDA_TRY(cudaMemcpyAsync(w.result_pin.p, p.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
+  if (recs)
+    XBFS_CUDA_TRY(cudaMemcpyAsync((void*)hrec, p.hist, sizeof(LevelRecDev) * kRecs, cudaMemcpyDeviceToHost, s));
   if (!lv_dev) XBFS_CUDA_TRY(cudaMemcpyAsync(levels, d_levels, (size_t)g->V * 4, cudaMemcpyDeviceToHost, s));
   if (parents && !par_dev)
     XBFS_CUDA_TRY(cudaMemcpyAsync(parents, d_parents, (size_t)g->V * 4, cudaMemcpyDeviceToHost, s));
@@ -3591,10 +3612,15 @@ xbfs_status bfs_single(Graph* g, int32_t src, int32_t* levels, int32_t* parents,
   XBFS_CUDA_TRY(cudaEventElapsedTime(&ms, w.ev0, w.ev1));
   XBFS_CUDA_TRY(cudaEventElapsedTime(&kms, w.evk0, w.ev1));
 
-  if (o.trace || stats) {
+  if (recs) {
     const int nl = std::min(hctl.depth, w.hist_cap);
-    std::vector<LevelRecDev> h(nl);
-    if (nl > 0) XBFS_CUDA_TRY(cudaMemcpy(h.data(), p.hist, sizeof(LevelRecDev) * nl, cudaMemcpyDeviceToHost));
+    std::vector<LevelRecDev> all;
+    const LevelRecDev* h = hrec;
+    if (nl > kRecs) {
+      all.resize(nl);
+      XBFS_CUDA_TRY(cudaMemcpy(all.data(), p.hist, sizeof(LevelRecDev) * nl, cudaMemcpyDeviceToHost));
+      h = all.data();
+    }
     w.trace.resize(nl);
     for (int i = 0; i < nl; ++i) {
       w.trace[i].level = i;
@@ -3720,8 +3746,9 @@ xbfs_status bfs_many(Graph* g, const int32_t* srcs, int32_t n, int32_t* levels, 
   }
   if (!dev_out && (st = copy_out(n - 1))) return st;
   XBFS_CUDA_TRY(cudaEventRecord(w.ev1, s));
-  std::vector<Ctl> hctl((size_t)n);
-  XBFS_CUDA_TRY(cudaMemcpyAsync(hctl.data(), w.ctl_log.p, sizeof(Ctl) * (size_t)n, cudaMemcpyDeviceToHost, s));
+  if ((st = w.result_pin.ensure(sizeof(Ctl) * (size_t)n))) return st;
+  const Ctl* hctl = w.result_pin.as<Ctl>();
+  XBFS_CUDA_TRY(cudaMemcpyAsync(w.result_pin.p, w.ctl_log.p, sizeof(Ctl) * (size_t)n, cudaMemcpyDeviceToHost, s));
   XBFS_CUDA_TRY(cudaStreamSynchronize(s));
   if (!dev_out) XBFS_CUDA_TRY(cudaStreamSynchronize(w.copy_stream));
   long long reached = 0, msum = 0, n_async = 0;
