@@ -549,7 +549,7 @@ def batched_roofline(V, E, n, ms):
     ach = b_alg / (ms * 1e-3) / 1e9
     return {"bound": "hbm", "achieved": round(ach, 1), "peak": peak, "unit": "GB/s", "frac": round(ach / peak, 4),
             "peak_source": peak_kind, "algorithmic_bytes_per_call": b_alg,
-            "kernel": "ms::k_msbfs + ms::k_ms_transpose (device time of the call)"}
+            "kernel": "ms::k_msbfs + ms::k_ms_expand (device time of the call)"}
 
 
 def extra_batched_same_graph(args, g, beg, plain_gteps, wname):
