@@ -3746,9 +3746,8 @@ xbfs_status bfs_many(Graph* g, const int32_t* srcs, int32_t n, int32_t* levels, 
   }
   if (!dev_out && (st = copy_out(n - 1))) return st;
   XBFS_CUDA_TRY(cudaEventRecord(w.ev1, s));
-  if ((st = w.result_pin.ensure(sizeof(Ctl) * (size_t)n))) return st;
-  const Ctl* hctl = w.result_pin.as<Ctl>();
-  XBFS_CUDA_TRY(cudaMemcpyAsync(w.result_pin.p, w.ctl_log.p, sizeof(Ctl) * (size_t)n, cudaMemcpyDeviceToHost, s));
+  std::vector<Ctl> hctl((size_t)n);
+  XBFS_CUDA_TRY(cudaMemcpyAsync(hctl.data(), w.ctl_log.p, sizeof(Ctl) * (size_t)n, cudaMemcpyDeviceToHost, s));
   XBFS_CUDA_TRY(cudaStreamSynchronize(s));
   if (!dev_out) XBFS_CUDA_TRY(cudaStreamSynchronize(w.copy_stream));
   long long reached = 0, msum = 0, n_async = 0;
