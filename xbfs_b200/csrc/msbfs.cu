@@ -971,13 +971,19 @@ __device__ __forceinline__ void expand_word(const u64* pl, size_t pstride, u64 v
 // rows of R-MAT scale 22: 8.6 GB written, 1.1 GB read), and those by how many
 // rows are written side by side: one CTA of 512 threads per SM that keeps to
 // one row takes 1.6 ms, four CTAs of 256 free-running threads 1.9, eight 2.6.
+//
+// The largest level is depth - 1 where every reached vertex has an edge, as on
+// a symmetric CSR. On a directed one the last frontier may reach only vertices
+// without out-edges, which get level `depth` and form no frontier of their own;
+// that level was processed, so the plane of its top bit has been zeroed.
 __global__ void __launch_bounds__(kExpand, 1)
     k_ms_expand(const u64* vis, const u64* lo, const u64* hi, int W, size_t ps, long long V, const long long* beg, int n,
-                int* out, size_t stride, Ctl* ctl) {
+                int* out, size_t stride, int symmetric, Ctl* ctl) {
   __shared__ long long red[kExpand / 32 + 1];
   const int depth = ctl->depth;
   if (depth == 0 && (ctl->more || ctl->bar.err)) return;
-  const int P = depth > 2 ? 32 - __clz(depth - 1) : 1;
+  const int top = symmetric ? depth - 1 : depth;  // no level is above it
+  const int P = top > 1 ? 32 - __clz(top) : 1;
   const long long v = blockIdx.x * (long long)kExpand + threadIdx.x;
   const bool in = v < V;
   long long reached = 0;
@@ -1192,7 +1198,7 @@ static xbfs_status run_pass(Graph* g, const int32_t* srcs, int n, int* d_out, si
     void* args[] = {&p};
     XBFS_CUDA_TRY(cudaLaunchCooperativeKernel(kfn, dim3(nsm * per_sm), dim3(ms::kBlock), args, smem, s));
     ms::k_ms_expand<<<(unsigned)((V + ms::kExpand - 1) / ms::kExpand), ms::kExpand, 0, s>>>(
-        p.vis, p.lo, p.hi, W, p.ps, V, p.beg, n, d_out, out_stride, p.ctl);
+        p.vis, p.lo, p.hi, W, p.ps, V, p.beg, n, d_out, out_stride, p.symmetric, p.ctl);
     XBFS_CUDA_TRY(cudaGetLastError());
     XBFS_CUDA_TRY(cudaMemcpyAsync(&hc, p.ctl, sizeof(hc), cudaMemcpyDeviceToHost, s));
     XBFS_CUDA_TRY(cudaStreamSynchronize(s));
