@@ -1097,11 +1097,13 @@ struct MsLease {
   }
 };
 
-// Grows b to n bytes; a buffer that was re-allocated is not clean any more.
+// Grows b to n bytes; a buffer that was re-allocated is not clean any more. Its
+// size tells, not its address: an allocation may get the place of the smaller one
+// just freed (16 bytes and then up to 512 always do).
 xbfs_status grow(DevBuf& b, size_t n, MsWorkspace& w) {
-  void* before = b.p;
+  const size_t before = b.bytes;
   const xbfs_status st = b.ensure(n);
-  if (b.p != before) w.clean = false;
+  if (b.bytes != before) w.clean = false;
   return st;
 }
 }  // namespace
