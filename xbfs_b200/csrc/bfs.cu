@@ -288,6 +288,15 @@ struct FewSure {
   float g_lo, g_hi;                 // vertices + 1 over the level before's
 };
 constexpr int kFewRing = 16;
+// Several CTAs decide a level by the box in force kFewLag levels before it: the
+// newest that all are sure to have (a box takes 1.8 us to draw, a level of
+// several CTAs 2.8 and more). An older box is left sooner and the network
+// evaluated in its stead: on 27 to 101 of the 830 to 1202 levels of a 1024 x 512
+// grid with 1, on 192 to 276 with 4; with 2 the grid takes 2.5% longer.
+constexpr unsigned kFewLag = 1;
+constexpr unsigned kFewLagSolo = 5;  // one CTA takes the newest box, at most this old
+constexpr int kFewBoxes = 8;
+static_assert(kFewLagSolo + 2 <= kFewBoxes && kFewLag <= kFewLagSolo, "a box is read while that many newer ones are drawn");
 
 // Per-CTA loop state owned by thread 0 (in shared memory).
 struct LoopState {
@@ -346,8 +355,8 @@ struct __align__(16) Smem {
   // is over) and the one it has dealt with
   unsigned few_rec[kFewRing][5];
   volatile unsigned few_seq, few_seen;
-  FewSure few_sure[2];          // what that warp is sure of, by the parity of few_made
-  volatile unsigned few_made;
+  FewSure few_sure[kFewBoxes];  // what that warp is sure of: rings of the boxes it drew, by their number,
+  volatile unsigned few_box_no[kFewBoxes];  // and of the number of the box in force after a level, by level
   __align__(16) float few_act[32];  // its evaluation's activations and statistics
   float few_raw[8];
   float few_margin;
@@ -2515,8 +2524,8 @@ struct FewStat {
 // network is sure to pick XBFS_TD_QUEUE: the margin of its decision is spread
 // over the features (see mlp_reuse_bound), of which the first five may each
 // move by the relative amount r, and the growth and the mean degree, which
-// hardly change in a run, by r / 4. Called by a full warp; `sure` in, the new
-// box (of nothing when the margin is used up) out.
+// hardly change in a run, by r / 4. Called by a full warp; returns a box of
+// nothing when the margin is used up (or is no number).
 __device__ __noinline__ FewSure few_box(const Params& p, Smem& sm, const FewStat& t) {
   const int lane = threadIdx.x & 31;
   const float n = (float)t.n, m = (float)t.m, n_u = (float)max(p.n_ni - (long long)t.vn, 0ll),
@@ -2539,8 +2548,9 @@ __device__ __noinline__ FewSure few_box(const Params& p, Smem& sm, const FewStat
   const float* q = sm.mlp_q;
   const float w = q[0] + q[1] + q[2] + q[3] + q[4] + 0.25f * (q[6] + q[7]);
   const float margin = sm.few_dec == XBFS_TD_QUEUE ? sm.few_margin : 0.f;
-  const float r = w > 0.f ? fminf(0.95f * (margin - 1e-5f) / (1.02f * w), 0.2f) : 0.f;
-  if (!(r > 1e-5f)) return FewSure{1u, 0u, 0u, 0u, 0u, 0u, 0u, 0.f, 0.f, 0.f, 0.f};
+  float r = 0.95f * (margin - 1e-5f) / (1.02f * w);
+  if (!(w > 0.f && r > 1e-5f)) return FewSure{1u, 0u, 0u, 0u, 0u, 0u, 0u, 0.f, 0.f, 0.f, 0.f};
+  r = fminf(r, 0.2f);
   // within r of c: (u - c) / (1 + c) <= r upwards, (c - u) / (1 + u) <= r
   // downwards; the growth's logarithm moves by at most |u - c| / min(u, c)
   const float down = 1.f / (1.f + r), r4 = 0.25f * r, down4 = 1.f / (1.f + r4);
@@ -2573,18 +2583,22 @@ __device__ __forceinline__ bool few_inside(const FewSure& b, unsigned n, unsigne
 // levels' records; with the learned switch it keeps a box (few_box) drawn around
 // a recent level, so that warp 0 seldom has to evaluate the network between
 // two levels. It follows warp 0 through few_seq and takes no part in the
-// levels' barriers.
+// levels' barriers. When it draws depends on the levels' statistics alone, not
+// on how far warp 0 is, and warp 0 of several CTAs decides by the box in force
+// kFewLag levels before the running one (few_box_no): all decide by the same box,
+// so none leaves the run while another stays, whatever the weights.
 template <bool MLP>
 __device__ __noinline__ void few_aside(const Params& p, Smem& sm, unsigned L0) {
   const int lane = threadIdx.x & 31;
   const bool records = blockIdx.x == 0;
-  FewSure b{1u, 0u, 0u, 0u, 0u, 0u, 0u, 0.f, 0.f, 0.f, 0.f};
-  FewSure h = b;  // the part of it after which a new one is drawn
+  FewSure h{1u, 0u, 0u, 0u, 0u, 0u, 0u, 0.f, 0.f, 0.f, 0.f};  // the part of the box after which a new one is drawn
   unsigned made = 0;
   for (unsigned next = L0 + 1;; ++next) {
+    // lane 0's look is every lane's, so that the warp goes on or ends together
+    // (a loop of lane 0 alone leaves the warp split: 4.2 us to draw a box, not 1.8)
     unsigned seq;
     for (;;) {
-      seq = sm.few_seq;
+      seq = __shfl_sync(0xffffffffu, sm.few_seq, 0);
       if (seq == ~0u || (int)(seq - next) >= 0) break;
       __nanosleep(40);
     }
@@ -2606,26 +2620,27 @@ __device__ __noinline__ void few_aside(const Params& p, Smem& sm, unsigned L0) {
         p.hist[next - 1].t1 = r.t0;
       }
     }
-    if (MLP && seq == next && !few_inside(h, t.n, t.m, t.vn, t.vm, t.level, t.prev)) {
-      b = few_box(p, sm, t);
-      h = b;
-      if (b.n_hi >= b.n_lo) {
-        h.n_lo = t.n - (t.n - min(b.n_lo, t.n)) / 2;
-        h.n_hi = t.n + (b.n_hi - t.n) / 2;
-        h.m_lo = t.m - (t.m - min(b.m_lo, t.m)) / 2;
-        h.m_hi = t.m + (b.m_hi - t.m) / 2;
-        h.vn_hi = t.vn + (b.vn_hi - t.vn) / 2;
-        h.vm_hi = t.vm + (b.vm_hi - t.vm) / 2;
-        h.level_hi = t.level + (b.level_hi - t.level) / 2;
+    if (MLP) {
+      // several CTAs: at every level that leaves h; one alone: unless it is behind
+      if ((sm.few > 1 || seq == next) && __any_sync(0xffffffffu, !few_inside(h, t.n, t.m, t.vn, t.vm, t.level, t.prev))) {
+        const FewSure b = few_box(p, sm, t);
+        h = b;
+        if (b.n_hi >= b.n_lo) {
+          h.n_lo = t.n - (t.n - min(b.n_lo, t.n)) / 2;
+          h.n_hi = t.n + (b.n_hi - t.n) / 2;
+          h.m_lo = t.m - (t.m - min(b.m_lo, t.m)) / 2;
+          h.m_hi = t.m + (b.m_hi - t.m) / 2;
+          h.vn_hi = t.vn + (b.vn_hi - t.vn) / 2;
+          h.vm_hi = t.vm + (b.vm_hi - t.vm) / 2;
+          h.level_hi = t.level + (b.level_hi - t.level) / 2;
+        }
+        ++made;
+        if (lane == 0) sm.few_sure[made % kFewBoxes] = b;
       }
-      __syncwarp();
       if (lane == 0) {
-        // warp 0 reads the other buffer until few_made moves on
-        sm.few_sure[(made + 1) & 1] = b;
+        sm.few_box_no[next % kFewBoxes] = made;
         __threadfence_block();
-        sm.few_made = made + 1;
       }
-      ++made;
     }
     __syncwarp();
     if (lane == 0) sm.few_seen = next;
@@ -2745,7 +2760,7 @@ __device__ __noinline__ bool small_levels(const Params& p, Smem& sm, long long L
     __syncthreads();
     if (threadIdx.x == 0) {
       sm.few_seq = sm.few_seen = (unsigned)L;
-      sm.few_made = 0;
+      for (int i = 0; i < kFewBoxes; ++i) sm.few_box_no[i] = 0;
       sm.few_sure[0] = FewSure{1u, 0u, 0u, 0u, 0u, 0u, 0u, 0.f, 0.f, 0.f, 0.f};
     }
     __syncthreads();
@@ -2767,17 +2782,25 @@ __device__ __noinline__ bool small_levels(const Params& p, Smem& sm, long long L
       for (;;) {
         const int par = (int)(L & 1);
         if (LEARNED && threadIdx.x < 32) {
-          // the box as it is now, while the others claim, as ranges of the
-          // next level's two counts: what it says of the visited sums, the
-          // level and the growth becomes part of n's and m's
-          const unsigned made = sm.few_made;
-          sure = sm.few_sure[made & 1];
+          // the box in force, while the others claim, as ranges of the next
+          // level's two counts: what it says of the visited sums, the level
+          // and the growth becomes part of n's and m's. One CTA takes the
+          // newest; several wait for the one of the level before.
+          unsigned at;
+          for (;;) {
+            at = __shfl_sync(0xffffffffu, sm.few_seen, 0);
+            if ((int)(at + (N > 1 ? kFewLag : kFewLagSolo) - st.level) >= 0) break;
+            __nanosleep(20);
+          }
+          __threadfence_block();
+          if (N > 1) at = st.level - L0 > kFewLag ? st.level - kFewLag : L0;
+          sure = sm.few_sure[at == L0 ? 0u : sm.few_box_no[at % kFewBoxes] % kFewBoxes];
           const float grown = (float)st.n + 1.f;
           sure.n_lo = max(sure.n_lo, (unsigned)fmaxf(ceilf(sure.g_lo * grown - 1.f), 0.f));
           sure.n_hi = min(min(sure.n_hi, (unsigned)fmaxf(sure.g_hi * grown - 1.f, 0.f)),
                           max(sure.vn_hi, st.vn) - st.vn);
           sure.m_hi = min(sure.m_hi, max(sure.vm_hi, st.vm) - st.vm);
-          if (sm.few_made != made || st.level + 1 > sure.level_hi) sure.n_lo = ~0u;  // being drawn anew, or left
+          if (st.level + 1 > sure.level_hi) sure.n_lo = ~0u;  // left
         }
         if (threadIdx.x >= 32 && (e0 & ~31u) < m) {  // whole warps
           for (unsigned e = e0;;) {
