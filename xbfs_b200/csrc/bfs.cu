@@ -2884,9 +2884,9 @@ __device__ __noinline__ bool small_levels(const Params& p, Smem& sm, long long L
         ls.ps = ps;
         ls.ps.n_prev = st.n;
         sm.red4[0] = L;
-        sm.few_rec[0][0] = m;
-        // the last warp may still have records to write
+        // the last warp may still have records to write, from any slot of its ring
         while ((int)(st.level - sm.few_seen) > 0) __nanosleep(20);
+        sm.few_rec[0][0] = m;
         sm.few_seq = ~0u;
       }
     }
