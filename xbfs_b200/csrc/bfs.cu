@@ -3542,6 +3542,62 @@ static xbfs_status init_state(Graph* g, const Params& p, int src, bool par_on, c
   return XBFS_OK;
 }
 
+// Pinned memory that a single call reads its results back into: the control block
+// and the first levels' records. A call takes an idle block or allocates one, and
+// gives it back when its copies have landed, so calls of several threads and
+// streams never share one; kIdleResults stay allocated for the process.
+// A block per graph handle made every handle's first call pay for pinning
+// (R-MAT scale 12: 2.4 ms in place of 0.56, as long as no other pinned memory was
+// alive); pageable memory costs a call with host levels 5 us (scale 10: 117 against
+// 112), since its copies wait for one another.
+constexpr int kResultRecs = 64;
+constexpr int kIdleResults = 2;
+struct ResultBlock {
+  Ctl ctl;
+  LevelRecDev rec[kResultRecs];
+};
+static std::mutex g_result_mu;
+static ResultBlock* g_result_idle[kIdleResults];
+
+namespace {
+struct ResultLease {
+  ResultBlock* b = nullptr;
+  cudaStream_t s;
+  bool landed = false;  // no copy into the block is under way
+  explicit ResultLease(cudaStream_t stream) : s(stream) {}
+  ResultLease(const ResultLease&) = delete;
+  ResultLease& operator=(const ResultLease&) = delete;
+  xbfs_status take() {
+    {
+      std::lock_guard<std::mutex> lk(g_result_mu);
+      for (ResultBlock*& x : g_result_idle)
+        if (x && !b) std::swap(x, b);
+    }
+    if (b) {
+      // a block from before a reset of the device is gone with it
+      cudaPointerAttributes a;
+      if (cudaPointerGetAttributes(&a, b) == cudaSuccess && a.type == cudaMemoryTypeHost) return XBFS_OK;
+      cudaGetLastError();
+      b = nullptr;
+    }
+    const cudaError_t e = cudaMallocHost((void**)&b, sizeof(ResultBlock));
+    if (e == cudaSuccess) return XBFS_OK;
+    b = nullptr;
+    cudaGetLastError();
+    return set_error(XBFS_ERR_OOM, "cudaMallocHost(%zu): %s", sizeof(ResultBlock), cudaGetErrorString(e));
+  }
+  ~ResultLease() {
+    if (!b || (!landed && cudaStreamSynchronize(s) != cudaSuccess)) return;  // a faulted context: nothing to keep
+    {
+      std::lock_guard<std::mutex> lk(g_result_mu);
+      for (ResultBlock*& x : g_result_idle)
+        if (!x && b) std::swap(x, b);
+    }
+    if (b) cudaFreeHost(b);
+  }
+};
+}  // namespace
+
 xbfs_status bfs_single(Graph* g, int32_t src, int32_t* levels, int32_t* parents, const xbfs_opts* uopts,
                        xbfs_stats* stats) {
   const auto t_start = std::chrono::steady_clock::now();
@@ -3616,18 +3672,19 @@ xbfs_status bfs_single(Graph* g, int32_t src, int32_t* levels, int32_t* parents,
   XBFS_CUDA_TRY(cudaEventRecord(w.ev1, s));
   // results and the first levels' records come back together, into pinned
   // memory; deeper traversals' other records are fetched once the depth is known
-  constexpr int kRecs = 64;
-  if ((st = w.result_pin.ensure(sizeof(Ctl) + sizeof(LevelRecDev) * kRecs))) return st;
-  const Ctl& hctl = *w.result_pin.as<Ctl>();
-  const LevelRecDev* hrec = reinterpret_cast<const LevelRecDev*>(w.result_pin.as<char>() + sizeof(Ctl));
+  ResultLease res(s);
+  if ((st = res.take())) return st;
+  const Ctl& hctl = res.b->ctl;
   const bool recs = o.trace || stats;
-  XBFS_CUDA_TRY(cudaMemcpyAsync(w.result_pin.p, p.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
+  XBFS_CUDA_TRY(cudaMemcpyAsync(&res.b->ctl, p.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
   if (recs)
-    XBFS_CUDA_TRY(cudaMemcpyAsync((void*)hrec, p.hist, sizeof(LevelRecDev) * kRecs, cudaMemcpyDeviceToHost, s));
+    XBFS_CUDA_TRY(
+        cudaMemcpyAsync(res.b->rec, p.hist, sizeof(LevelRecDev) * kResultRecs, cudaMemcpyDeviceToHost, s));
   if (!lv_dev) XBFS_CUDA_TRY(cudaMemcpyAsync(levels, d_levels, (size_t)g->V * 4, cudaMemcpyDeviceToHost, s));
   if (parents && !par_dev)
     XBFS_CUDA_TRY(cudaMemcpyAsync(parents, d_parents, (size_t)g->V * 4, cudaMemcpyDeviceToHost, s));
   XBFS_CUDA_TRY(cudaStreamSynchronize(s));
+  res.landed = true;
   if (hctl.bar.err != 0)
     return set_error((xbfs_status)hctl.bar.err, "traversal kernel reported %s", xbfs_strerror(hctl.bar.err));
   w.last_levels = hctl.depth;
@@ -3638,8 +3695,8 @@ xbfs_status bfs_single(Graph* g, int32_t src, int32_t* levels, int32_t* parents,
   if (recs) {
     const int nl = std::min(hctl.depth, w.hist_cap);
     std::vector<LevelRecDev> all;
-    const LevelRecDev* h = hrec;
-    if (nl > kRecs) {
+    const LevelRecDev* h = res.b->rec;
+    if (nl > kResultRecs) {
       all.resize(nl);
       XBFS_CUDA_TRY(cudaMemcpy(all.data(), p.hist, sizeof(LevelRecDev) * nl, cudaMemcpyDeviceToHost));
       h = all.data();

@@ -71,7 +71,6 @@ struct SsWorkspace {
   // that copies finished level arrays out, and the events between the two
   DevBuf levels_tmp2;
   DevBuf ctl_log;          // Ctl of every traversal of one call
-  PinnedBuf result_pin;    // control block and level records of one call, read back
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t ev_done[2] = {nullptr, nullptr}, ev_copied[2] = {nullptr, nullptr};
   int grid = 0, block = 0;
