@@ -34,3 +34,24 @@ def test_first_single_call_of_a_handle():
             many.append(_us(lambda: g.bfs_many(src, levels=lv)))
         g.free()
     assert np.median(single) < 2 * np.median(many[1:])
+
+
+def test_first_batch_of_a_handle_and_its_end():
+    """With the last handle the batched workspace goes, and the next first call
+    allocates it again: together no more than what a pipelined call's workspace,
+    some 30 allocations, costs (2.3 ms against 5.9 when measured; 11.4 with an
+    allocation for every buffer)."""
+    import gc
+
+    import torch
+    gc.collect()
+    batch, many = [], []
+    for i in range(13):
+        g = Graph.rmat(18, 16, 5 + i)
+        srcs = pick_sources(g.offsets(), 64, 1)
+        lv = torch.empty((64, g.V), dtype=torch.int32, device="cuda:0")
+        if i % 2:
+            batch.append(_us(lambda: g.bfs_batch(srcs, levels=lv)) + _us(g.free))
+        else:
+            many.append(_us(lambda: g.bfs_many(srcs[:1], levels=lv[:1])) + _us(g.free))
+    assert np.median(batch) < 1.2 * np.median(many[1:])

@@ -1027,10 +1027,18 @@ __global__ void __launch_bounds__(kExpand, 1)
 // ---------------------------------------------------------------------------
 // Host driver
 // ---------------------------------------------------------------------------
+// One allocation holds all of a traversal's buffers but the upper level planes: an
+// allocation and its release take 0.3 ms and more each, whatever their size, and a
+// program that loads one graph after another pays both for every graph (R-MAT
+// scale 18, 64 sources: 5.6 -> 0.76 ms for the first call, 5.7 -> 1.6 to
+// free the graph, with 25 allocations and with one). What has to be zero when a
+// traversal starts comes first, in zero_bytes of its own, so that graphs and
+// words per vertex of other sizes find zeros wherever their buffers lie in it.
 struct MsWorkspace {
   int device = 0;
-  DevBuf vis, F[3], fbm[3], lo, hi, done, q[4], qe[4], qb[4], ctl, mega_v, tasks, mega_n, mega_acc;
-  bool clean = true;  // F, fbm, mega_n and mega_acc are all zero (what a finished traversal leaves)
+  DevBuf mem, hi;
+  size_t zero_bytes = 0;
+  bool clean = false;  // the first zero_bytes are all zero (what a finished traversal leaves)
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   ~MsWorkspace() {
     if (e0) cudaEventDestroy(e0);
@@ -1097,13 +1105,17 @@ struct MsLease {
   }
 };
 
-// Grows b to n bytes; a buffer that was re-allocated is not clean any more. Its
-// size tells, not its address: an allocation may get the place of the smaller one
-// just freed (16 bytes and then up to 512 always do).
-xbfs_status grow(DevBuf& b, size_t n, MsWorkspace& w) {
-  const size_t before = b.bytes;
-  const xbfs_status st = b.ensure(n);
-  if (b.bytes != before) w.clean = false;
+// Makes room for nz bytes that must be zero and n others. A new allocation is not
+// clean, wherever it lies: cudaMalloc may give it the place of the one just freed.
+xbfs_status grow(MsWorkspace& w, size_t nz, size_t n) {
+  if (w.mem.p && nz <= w.zero_bytes && n <= w.mem.bytes - w.zero_bytes) return XBFS_OK;
+  nz = std::max(nz, w.zero_bytes);
+  n = std::max(n, w.mem.bytes - w.zero_bytes);
+  w.clean = false;
+  w.zero_bytes = 0;
+  w.mem.release();
+  const xbfs_status st = w.mem.ensure(nz + n);
+  if (!st) w.zero_bytes = nz;
   return st;
 }
 }  // namespace
@@ -1121,23 +1133,28 @@ static xbfs_status run_pass(Graph* g, const int32_t* srcs, int n, int* d_out, si
   const size_t n_mega = bu ? (size_t)g->cnt_deg_gt[ms::kMegaLog] : 0;
   const size_t n_tasks = n_mega ? n_mega + ((size_t)g->E >> ms::kMegaLog) : 0;
   xbfs_status st;
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = at;
+    at += (bytes + 255) & ~(size_t)255;
+    return o;
+  };
   // the buffers that a finished traversal leaves all zero
   const size_t rows = words + 64;  // and one zero row past the last vertex
-  struct { DevBuf* b; size_t n; } zero[] = {{&w.F[0], rows}, {&w.F[1], rows}, {&w.F[2], rows}, {&w.fbm[0], bm},
-                                            {&w.fbm[1], bm}, {&w.fbm[2], bm}, {&w.mega_n, n_mega * 4},
-                                            {&w.mega_acc, n_mega * W * 8}};
-  for (auto& z : zero)
-    if ((st = grow(*z.b, z.n, w))) return st;
-  if ((st = w.vis.ensure(words)) || (st = w.lo.ensure(words * ms::kLoPlanes)) || (st = w.done.ensure(bm)) ||
-      (st = w.ctl.ensure(sizeof(ms::Ctl))) || (st = w.mega_v.ensure(n_mega * 4)) ||
-      (st = w.tasks.ensure(n_tasks * 8)))
-    return st;
-  for (int i = 0; i < 4; ++i)
-    if ((st = w.q[i].ensure((size_t)V * 4 + 4)) || (st = w.qe[i].ensure((size_t)V * 4 + 4)) ||
-        (st = w.qb[i].ensure((size_t)V * 4 + 4)))
-      return st;
-  if (!w.clean)
-    for (auto& z : zero) XBFS_CUDA_TRY(cudaMemsetAsync(z.b->p, 0, z.b->bytes, s));
+  size_t o_F[3], o_fbm[3], o_q[4][3];
+  for (auto& o : o_F) o = take(rows);
+  for (auto& o : o_fbm) o = take(bm);
+  const size_t o_mega_n = take(n_mega * 4), o_mega_acc = take(n_mega * W * 8);
+  const size_t nz = at;
+  at = 0;
+  const size_t o_vis = take(words), o_lo = take(words * ms::kLoPlanes), o_done = take(bm),
+               o_ctl = take(sizeof(ms::Ctl)), o_mega_v = take(n_mega * 4), o_tasks = take(n_tasks * 8);
+  for (auto& q : o_q)
+    for (auto& o : q) o = take((size_t)V * 4 + 4);
+  if ((st = grow(w, nz, at))) return st;
+  char* const zero = w.mem.as<char>();
+  char* const rest = zero + w.zero_bytes;
+  if (!w.clean) XBFS_CUDA_TRY(cudaMemsetAsync(zero, 0, w.zero_bytes, s));
   w.clean = false;  // until this traversal has finished
   ms::Params<W> p;
   memset(&p, 0, sizeof(p));
@@ -1145,24 +1162,24 @@ static xbfs_status run_pass(Graph* g, const int32_t* srcs, int n, int* d_out, si
   p.csr = g->csr.as<int>();
   p.V = V;
   p.E = g->E;
-  p.vis = w.vis.as<ms::u64>();
+  p.vis = reinterpret_cast<ms::u64*>(rest + o_vis);
   for (int i = 0; i < 3; ++i) {
-    p.F[i] = w.F[i].as<ms::u64>();
-    p.fbm[i] = w.fbm[i].as<uint32_t>();
+    p.F[i] = reinterpret_cast<ms::u64*>(zero + o_F[i]);
+    p.fbm[i] = reinterpret_cast<uint32_t*>(zero + o_fbm[i]);
   }
   p.ps = (long long)ps;
-  p.lo = w.lo.as<ms::u64>();
-  p.done = w.done.as<uint32_t>();
+  p.lo = reinterpret_cast<ms::u64*>(rest + o_lo);
+  p.done = reinterpret_cast<uint32_t*>(rest + o_done);
   for (int i = 0; i < 4; ++i) {
-    p.qids[i] = w.q[i].as<int>();
-    p.qeb[i] = w.qe[i].as<unsigned>();
-    p.qbg[i] = w.qb[i].as<unsigned>();
+    p.qids[i] = reinterpret_cast<int*>(rest + o_q[i][0]);
+    p.qeb[i] = reinterpret_cast<unsigned*>(rest + o_q[i][1]);
+    p.qbg[i] = reinterpret_cast<unsigned*>(rest + o_q[i][2]);
   }
-  p.mega_v = w.mega_v.as<int>();
-  p.tasks = w.tasks.as<uint2>();
-  p.mega_n = w.mega_n.as<unsigned>();
-  p.mega_acc = w.mega_acc.as<ms::u64>();
-  p.ctl = w.ctl.as<ms::Ctl>();
+  p.mega_v = reinterpret_cast<int*>(rest + o_mega_v);
+  p.tasks = reinterpret_cast<uint2*>(rest + o_tasks);
+  p.mega_n = reinterpret_cast<unsigned*>(zero + o_mega_n);
+  p.mega_acc = reinterpret_cast<ms::u64*>(zero + o_mega_acc);
+  p.ctl = reinterpret_cast<ms::Ctl*>(rest + o_ctl);
   p.nwords = nwords;
   p.m_active = g->E;
   // The single-source default (0.1) means "use the batched default". An edge
