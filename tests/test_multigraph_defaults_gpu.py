@@ -1,0 +1,47 @@
+"""Thresholds of a multi-graph launch before it is tuned: graphs that one CTA owns
+keep theirs whatever suits the teams of large graphs."""
+import numpy as np
+import pytest
+
+import oracle
+from xbfs_b200 import Graph, MultiGraph, pick_sources
+
+pytestmark = pytest.mark.gpu
+
+
+def _set(n, max_scale, max_vertices):
+    rng = np.random.default_rng(n)
+    half = n // 2
+    graphs = [Graph.rmat(int(rng.integers(10, max_scale + 1)), int(rng.integers(8, 33)), 1 + i) for i in range(half)]
+    graphs += [Graph.er(int(rng.integers(1000, max_vertices + 1)), 8.0, 1 + i) for i in range(half, n)]
+    srcs = np.array([pick_sources(g.offsets(), 1, i)[0] for i, g in enumerate(graphs)], dtype=np.int32)
+    return graphs, srcs
+
+
+def test_sets_of_small_graphs_before_tuning():
+    """No slower than with (32, 4), another configuration of one CTA, on a set that
+    takes 1.27 times as long with those of the teams (8, 14). The margin is three
+    times what medians of one side differ by (2%)."""
+    import torch
+    graphs, srcs = _set(30, 12, 8000)
+    default, given = MultiGraph(graphs), MultiGraph(graphs)
+    given.set_config(512, 32, 4.0)
+    ms = ([], [])
+    for _ in range(31):
+        for k, mg in enumerate((default, given)):
+            lv = torch.empty(mg.total_V, dtype=torch.int32, device="cuda:0")
+            ms[k].append(mg.bfs(srcs, levels=lv).device_ms)
+    assert np.median(ms[0]) < 1.06 * np.median(ms[1])
+
+
+def test_levels_with_both_kinds_of_graph_and_every_configuration():
+    graphs, srcs = _set(6, 11, 3000)
+    graphs += [Graph.rmat(14, 24, 3), Graph.er(60000, 8.0, 4)]   # teams'
+    srcs = np.concatenate([srcs, [pick_sources(g.offsets(), 1, 5)[0] for g in graphs[6:]]]).astype(np.int32)
+    refs = [oracle.bfs_queue(*g.download(), int(s)) for g, s in zip(graphs, srcs)]
+    mg = MultiGraph(graphs)
+    for cfg in (None, (256, 0, 0.5), (512, 5000, 14.0), (1024, 8, 1e-6), (512, 32, 4.0), (512, 8, 4.0), (512, 8, 14.0)):
+        if cfg:
+            mg.set_config(*cfg)
+        for ref, lv in zip(refs, mg.split(mg.bfs(srcs).levels)):
+            assert np.array_equal(lv, ref), cfg

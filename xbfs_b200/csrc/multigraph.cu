@@ -54,6 +54,12 @@ struct Team {
   unsigned long long n[4], m[4];  // frontier vertices, degree sum
 };
 
+struct Thresholds {
+  int thread_max;  // top-down: degree <= thread_max expanded by one lane
+  float alpha;     // bottom-up when m_f * alpha > m_u
+  bool operator==(const Thresholds& o) const { return thread_max == o.thread_max && alpha == o.alpha; }
+};
+
 struct Desc {
   long long b_off;   // offset of the graph's V+1 local offsets in the beg arena
   long long e_off;   // offset of its neighbours in the csr arena
@@ -80,8 +86,7 @@ struct Params {
   long long heavy_cap;
   int* err;               // status of the launch
   int smem_words;         // words per bitmap available in shared memory
-  int thread_max;         // top-down: degree <= thread_max expanded by one lane
-  float alpha;            // bottom-up when m_f * alpha > m_u
+  Thresholds single, by_team;  // of graphs owned by one CTA, and by a team
   unsigned long long* edges;  // per graph: sum of degrees of reached vertices
 };
 
@@ -159,7 +164,7 @@ __device__ bool team_bfs(const Params& p, Team* team, uint32_t* bits, int* heavy
       const long long n_f = (long long)ld_cg_u64(&team->n[L & 3]), m_f = (long long)ld_cg_u64(&team->m[L & 3]);
       *s_mu -= m_f;
       reached += (unsigned long long)m_f;
-      *s_decision = n_f == 0 ? -1 : ((double)m_f * (double)p.alpha > (double)*s_mu ? 1 : 0);
+      *s_decision = n_f == 0 ? -1 : ((double)m_f * (double)p.by_team.alpha > (double)*s_mu ? 1 : 0);
       if (rank == 0) {
         team->n[(L + 2) & 3] = team->m[(L + 2) & 3] = 0ull;
         team->heavy[(L + 2) & 3] = 0u;
@@ -249,13 +254,13 @@ __device__ bool team_bfs(const Params& p, Team* team, uint32_t* bits, int* heavy
           e1 = __ldg(beg + u + 1);
         }
         const long long deg = e1 - e0;
-        if (mine && deg <= p.thread_max)
+        if (mine && deg <= p.by_team.thread_max)
           for (long long e = e0; e < e1; e += 4) team_claim4(csr, e, 1, e1, vis, nxt, beg, lv, L + 1, my_n, my_m);
-        if (mine && deg > p.thread_max && deg > kHeavy) {
+        if (mine && deg > p.by_team.thread_max && deg > kHeavy) {
           const unsigned at = atomicAdd(hc, 1u);
           heavy[at] = u;
         }
-        unsigned mid = __ballot_sync(0xffffffffu, mine && deg > p.thread_max && deg <= kHeavy);
+        unsigned mid = __ballot_sync(0xffffffffu, mine && deg > p.by_team.thread_max && deg <= kHeavy);
         while (mid) {
           const int hl = __ffs(mid) - 1;
           mid &= mid - 1;
@@ -360,7 +365,7 @@ __global__ void __launch_bounds__(BLOCK) k_multi(Params p) {
     m_u -= m_f;
     int L = 0;
     while (n_f > 0) {
-      const bool bu = (double)m_f * (double)p.alpha > (double)m_u;
+      const bool bu = (double)m_f * (double)p.single.alpha > (double)m_u;
       long long my_n = 0, my_m = 0;
       if (!bu) {
         // top-down: warps take frontier words; light vertices one per lane,
@@ -375,7 +380,7 @@ __global__ void __launch_bounds__(BLOCK) k_multi(Params p) {
             e0 = __ldg(beg + u_l);
             e1 = __ldg(beg + u_l + 1);
           }
-          const bool light = mine && (e1 - e0) <= p.thread_max;
+          const bool light = mine && (e1 - e0) <= p.single.thread_max;
           if (light) {
             for (long long e = e0; e < e1; ++e) {
               const int v = __ldg(csr + e);
@@ -466,14 +471,17 @@ struct MultiGraph {
   cudaStream_t stream = nullptr;
   // tuned configuration
   int block = 512;
-  // before tuning; with 8 and 14 the 96-graph set takes 0.86 ms, with 32 and 4 1.40
-  int thread_max = 8;
-  float alpha = 14.f;
+  // Before tuning. Teams: with 8 and 14 a set of 96 graphs takes 0.86 ms, with 32
+  // and 4 1.40. One CTA: 30 graphs of up to 2^12 vertices take 218 us with 8 and
+  // 14, 171 with 32 and 4 and 155 with 8 and 4; 128 of them 267, 243 and 221; 12
+  // uniform random ones of 14,000 vertices 353, 320 and 289; 12 grids of 100 x 90
+  // 995, 855 and 883. A configuration that was tuned or set is both's.
+  mg::Thresholds single = {8, 4.f}, by_team = {8, 14.f};
   // captured replay
   cudaGraphExec_t exec = nullptr;
   int* exec_levels = nullptr;
-  int exec_block = 0, exec_thread_max = 0;
-  float exec_alpha = 0;
+  int exec_block = 0;
+  mg::Thresholds exec_single = {0, 0.f}, exec_by_team = {0, 0.f};
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   ~MultiGraph() {
     DeviceGuard dg(device);
@@ -493,7 +501,8 @@ static_assert(mg::kBig <= 32ll * kSmemWords, "graphs too large for shared memory
 // the teams. What lies before the teams is copied to the host after it.
 constexpr size_t kCtlEdges = 64;
 
-static xbfs_status enqueue_multi(MultiGraph* m, int* d_levels, int block, int thread_max, float alpha) {
+static xbfs_status enqueue_multi(MultiGraph* m, int* d_levels, int block, const mg::Thresholds& single,
+                                 const mg::Thresholds& by_team) {
   cudaStream_t s = m->stream;
   XBFS_CUDA_TRY(cudaMemsetAsync(d_levels, 0xff, (size_t)m->total_V * 4, s));
   XBFS_CUDA_TRY(cudaMemsetAsync(m->ctl.p, 0, m->ctl.bytes, s));
@@ -515,8 +524,8 @@ static xbfs_status enqueue_multi(MultiGraph* m, int* d_levels, int block, int th
   p.heavy = m->heavy.as<int>();
   p.heavy_cap = m->heavy_cap;
   p.smem_words = kSmemWords;
-  p.thread_max = thread_max;
-  p.alpha = alpha;
+  p.single = single;
+  p.by_team = by_team;
   p.edges = reinterpret_cast<unsigned long long*>(m->ctl.as<char>() + kCtlEdges);
   const size_t smem = (size_t)3 * p.smem_words * 4;
   int nsm = 148;
@@ -556,10 +565,11 @@ __global__ void k_mg_set_sources(mg::Desc* desc, const int* srcs, int n) {
 // One call: copy sources, patch descriptors, reset outputs, run. Captured into
 // a CUDA graph on first use and replayed while the output pointer and the
 // configuration stay the same.
-static xbfs_status run_multi(MultiGraph* m, int* d_levels, int block, int thread_max, float alpha, float* ms_out) {
+static xbfs_status run_multi(MultiGraph* m, int* d_levels, int block, const mg::Thresholds& single,
+                             const mg::Thresholds& by_team, float* ms_out) {
   cudaStream_t s = m->stream;
   const bool reuse = m->exec && m->exec_levels == d_levels && m->exec_block == block &&
-                     m->exec_thread_max == thread_max && m->exec_alpha == alpha;
+                     m->exec_single == single && m->exec_by_team == by_team;
   if (!reuse) {
     if (m->exec) {
       cudaGraphExecDestroy(m->exec);
@@ -575,7 +585,7 @@ static xbfs_status run_multi(MultiGraph* m, int* d_levels, int block, int thread
         e = cudaGetLastError();
       }
       if (e != cudaSuccess) st = set_error(XBFS_ERR_CUDA, "capture: %s", cudaGetErrorString(e));
-      if (!st) st = enqueue_multi(m, d_levels, block, thread_max, alpha);
+      if (!st) st = enqueue_multi(m, d_levels, block, single, by_team);
       if (!st) {
         e = cudaMemcpyAsync(m->ctl_pin.p, m->ctl.p, m->ctl_teams, cudaMemcpyDeviceToHost, s);
         if (e != cudaSuccess) st = set_error(XBFS_ERR_CUDA, "capture: %s", cudaGetErrorString(e));
@@ -592,8 +602,8 @@ static xbfs_status run_multi(MultiGraph* m, int* d_levels, int block, int thread
     XBFS_CUDA_TRY(ie);
     m->exec_levels = d_levels;
     m->exec_block = block;
-    m->exec_thread_max = thread_max;
-    m->exec_alpha = alpha;
+    m->exec_single = single;
+    m->exec_by_team = by_team;
   }
   XBFS_CUDA_TRY(cudaEventRecord(m->e0, s));
   XBFS_CUDA_TRY(cudaGraphLaunch(m->exec, s));
@@ -715,7 +725,7 @@ xbfs_status xbfs_multi_bfs(xbfs_multi* mh, const int32_t* srcs, int32_t* levels,
     d_levels = m->levels_tmp.as<int>();
   }
   float ms = 0;
-  if ((st = run_multi(m, d_levels, m->block, m->thread_max, m->alpha, &ms))) return st;
+  if ((st = run_multi(m, d_levels, m->block, m->single, m->by_team, &ms))) return st;
   if (!dev) XBFS_CUDA_TRY(cudaMemcpy(levels, d_levels, (size_t)m->total_V * 4, cudaMemcpyDeviceToHost));
   if (stats) {
     const unsigned long long* e = reinterpret_cast<unsigned long long*>(m->ctl_pin.as<char>() + kCtlEdges);
@@ -746,8 +756,8 @@ xbfs_status xbfs_multi_tune(xbfs_multi* mh, const int32_t* srcs, int32_t reps, i
   const int tms[] = {8, 32, 128};
   const float alphas[] = {2.f, 4.f, 14.f};
   float best = 1e30f;
-  int bb = m->block, bt = m->thread_max;
-  float ba = m->alpha;
+  int bb = m->block;
+  mg::Thresholds best_th = m->single;
   if (reps < 1) reps = 1;
   for (int b : blocks)
     for (int t : tms)
@@ -755,23 +765,21 @@ xbfs_status xbfs_multi_tune(xbfs_multi* mh, const int32_t* srcs, int32_t reps, i
         float tot = 0;
         for (int r = 0; r < reps + 1; ++r) {
           float ms = 0;
-          if ((st = run_multi(m, m->levels_tmp.as<int>(), b, t, a, &ms))) return st;
+          if ((st = run_multi(m, m->levels_tmp.as<int>(), b, {t, a}, {t, a}, &ms))) return st;
           if (r > 0) tot += ms;  // first run builds the graph
         }
         tot /= reps;
         if (tot < best) {
           best = tot;
           bb = b;
-          bt = t;
-          ba = a;
+          best_th = {t, a};
         }
       }
   m->block = bb;
-  m->thread_max = bt;
-  m->alpha = ba;
+  m->single = m->by_team = best_th;
   if (block_out) *block_out = bb;
-  if (thread_max_out) *thread_max_out = bt;
-  if (alpha_out) *alpha_out = ba;
+  if (thread_max_out) *thread_max_out = best_th.thread_max;
+  if (alpha_out) *alpha_out = best_th.alpha;
   if (best_ms_out) *best_ms_out = best;
   return XBFS_OK;
 }
@@ -782,8 +790,7 @@ xbfs_status xbfs_multi_set_config(xbfs_multi* mh, int32_t block, int32_t thread_
   if (block != 256 && block != 512 && block != 1024) return set_error(XBFS_ERR_INVALID_ARG, "block must be 256/512/1024");
   if (thread_max < 0 || !(alpha > 0)) return set_error(XBFS_ERR_INVALID_ARG, "bad threshold");
   m->block = block;
-  m->thread_max = thread_max;
-  m->alpha = alpha;
+  m->single = m->by_team = {thread_max, alpha};
   return XBFS_OK;
 }
 
