@@ -255,8 +255,10 @@ xbfs_status xbfs_multi_info(const xbfs_multi* m, int64_t* total_V, int64_t* tota
 xbfs_status xbfs_multi_bfs(xbfs_multi* m, const int32_t* srcs, int32_t* levels, const xbfs_opts* opts,
                            xbfs_stats* stats);
 /* Autotuner: times every candidate (threads per CTA 256/512/1024, thread/warp
- * degree threshold, direction threshold) on these sources and keeps the
- * fastest for later xbfs_multi_bfs calls. */
+ * degree threshold, direction threshold) and the configuration that is there
+ * on these sources and keeps the fastest for later xbfs_multi_bfs calls. (Before
+ * tuning, large and small graphs have thresholds of their own; if that stays the
+ * fastest, the small ones' are reported.) */
 xbfs_status xbfs_multi_tune(xbfs_multi* m, const int32_t* srcs, int32_t reps, int32_t* block,
                             int32_t* thread_max, float* alpha, float* best_ms);
 xbfs_status xbfs_multi_set_config(xbfs_multi* m, int32_t block, int32_t thread_max, float alpha);

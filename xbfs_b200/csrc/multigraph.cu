@@ -743,7 +743,8 @@ xbfs_status xbfs_multi_bfs(xbfs_multi* mh, const int32_t* srcs, int32_t* levels,
 
 // Autotuner: times every (threads per CTA, thread/warp degree threshold,
 // direction threshold) candidate on the caller's sources and keeps the
-// fastest. Returns the chosen configuration.
+// fastest. Returns the chosen configuration, of the two kinds of graph the one of
+// single CTAs where they differ.
 xbfs_status xbfs_multi_tune(xbfs_multi* mh, const int32_t* srcs, int32_t reps, int32_t* block_out,
                             int32_t* thread_max_out, float* alpha_out, float* best_ms_out) {
   MultiGraph* m = (MultiGraph*)mh;
@@ -757,29 +758,37 @@ xbfs_status xbfs_multi_tune(xbfs_multi* mh, const int32_t* srcs, int32_t reps, i
   const float alphas[] = {2.f, 4.f, 14.f};
   float best = 1e30f;
   int bb = m->block;
-  mg::Thresholds best_th = m->single;
+  mg::Thresholds bs = m->single, bt = m->by_team;
   if (reps < 1) reps = 1;
+  auto time_one = [&](int b, const mg::Thresholds& single, const mg::Thresholds& by_team) -> xbfs_status {
+    float tot = 0;
+    for (int r = 0; r < reps + 1; ++r) {
+      float ms = 0;
+      if (xbfs_status e = run_multi(m, m->levels_tmp.as<int>(), b, single, by_team, &ms)) return e;
+      if (r > 0) tot += ms;  // first run builds the graph
+    }
+    tot /= reps;
+    if (tot < best) {
+      best = tot;
+      bb = b;
+      bs = single;
+      bt = by_team;
+    }
+    return XBFS_OK;
+  };
+  // the configuration that is there, whose two kinds of graph may differ, then
+  // every common one
+  if ((st = time_one(m->block, m->single, m->by_team))) return st;
   for (int b : blocks)
     for (int t : tms)
-      for (float a : alphas) {
-        float tot = 0;
-        for (int r = 0; r < reps + 1; ++r) {
-          float ms = 0;
-          if ((st = run_multi(m, m->levels_tmp.as<int>(), b, {t, a}, {t, a}, &ms))) return st;
-          if (r > 0) tot += ms;  // first run builds the graph
-        }
-        tot /= reps;
-        if (tot < best) {
-          best = tot;
-          bb = b;
-          best_th = {t, a};
-        }
-      }
+      for (float a : alphas)
+        if ((st = time_one(b, {t, a}, {t, a}))) return st;
   m->block = bb;
-  m->single = m->by_team = best_th;
+  m->single = bs;
+  m->by_team = bt;
   if (block_out) *block_out = bb;
-  if (thread_max_out) *thread_max_out = best_th.thread_max;
-  if (alpha_out) *alpha_out = best_th.alpha;
+  if (thread_max_out) *thread_max_out = bs.thread_max;
+  if (alpha_out) *alpha_out = bs.alpha;
   if (best_ms_out) *best_ms_out = best;
   return XBFS_OK;
 }
