@@ -39,7 +39,7 @@ def test_first_single_call_of_a_handle():
 def test_first_batch_of_a_handle_and_its_end():
     """With the last handle the batched workspace goes, and the next first call
     allocates it again: together no more than what a pipelined call's workspace,
-    some 30 allocations, costs (2.3 ms against 5.9 when measured; 11.4 with an
+    some 30 allocations, costs (3.0 ms against 5.9 when measured; 11.4 with an
     allocation for every buffer)."""
     import gc
 

@@ -19,12 +19,12 @@
 //    API (four levels per step, spread to bytes by a multiply).
 //  * Bottom-up takes W/2 lanes per vertex, two words (16 bytes) each: a
 //    warp reads 8 (W = 8) to 32 neighbours' frontier words per load
-//    instruction as whole sectors, four loads in flight. Low-degree vertices
-//    of a ticket's vertices stream through the lane groups from a per-warp
-//    list, higher degrees take a whole warp, and the neighbour lists of
-//    degree above kMega are cut into chunks that any warp of the grid takes,
-//    their gains meeting in an accumulator that the chunk finishing last
-//    merges.
+//    instruction as whole sectors, eight loads in flight (four for high-degree
+//    vertices below W = 8). Low-degree vertices of a ticket stream through the
+//    lane groups from a per-warp list, higher degrees take a whole warp, and
+//    the neighbour lists of degree above kMega are cut into chunks that any
+//    warp of the grid takes, their gains meeting in an accumulator that the
+//    chunk finishing last merges.
 //  * Only sources that are alive (some vertex gained them at the last
 //    level) are searched for: a source whose component is exhausted stops
 //    holding up the early exit of every other vertex.
@@ -1027,18 +1027,18 @@ __global__ void __launch_bounds__(kExpand, 1)
 // ---------------------------------------------------------------------------
 // Host driver
 // ---------------------------------------------------------------------------
-// One allocation holds all of a traversal's buffers but the upper level planes: an
+// Two allocations hold a traversal's buffers, the upper level planes excepted: an
 // allocation and its release take 0.3 ms and more each, whatever their size, and a
 // program that loads one graph after another pays both for every graph (R-MAT
-// scale 18, 64 sources: 5.6 -> 0.76 ms for the first call, 5.7 -> 1.6 to
-// free the graph, with 25 allocations and with one). What has to be zero when a
-// traversal starts comes first, in zero_bytes of its own, so that graphs and
-// words per vertex of other sizes find zeros wherever their buffers lie in it.
+// scale 18, 64 sources: 5.7 -> 1.1 ms for the first call, 5.7 -> 1.9 to
+// free the graph, with 25 allocations and with two). What has to be zero when a
+// traversal starts lies in one of its own, so that graphs and words per vertex of
+// other sizes find zeros wherever their buffers are in it. (With both in one
+// allocation 512 sources on R-MAT scale 21 took 3.334 ms, not 3.316.)
 struct MsWorkspace {
   int device = 0;
-  DevBuf mem, hi;
-  size_t zero_bytes = 0;
-  bool clean = false;  // the first zero_bytes are all zero (what a finished traversal leaves)
+  DevBuf zero, rest, hi;
+  bool clean = false;  // `zero` is all zero (what a finished traversal leaves)
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   ~MsWorkspace() {
     if (e0) cudaEventDestroy(e0);
@@ -1104,20 +1104,6 @@ struct MsLease {
     if (have < kMsIdle && g_ms_graphs > 0) idle.push_back(std::move(w));
   }
 };
-
-// Makes room for nz bytes that must be zero and n others. A new allocation is not
-// clean, wherever it lies: cudaMalloc may give it the place of the one just freed.
-xbfs_status grow(MsWorkspace& w, size_t nz, size_t n) {
-  if (w.mem.p && nz <= w.zero_bytes && n <= w.mem.bytes - w.zero_bytes) return XBFS_OK;
-  nz = std::max(nz, w.zero_bytes);
-  n = std::max(n, w.mem.bytes - w.zero_bytes);
-  w.clean = false;
-  w.zero_bytes = 0;
-  w.mem.release();
-  const xbfs_status st = w.mem.ensure(nz + n);
-  if (!st) w.zero_bytes = nz;
-  return st;
-}
 }  // namespace
 
 template <int W>
@@ -1151,10 +1137,13 @@ static xbfs_status run_pass(Graph* g, const int32_t* srcs, int n, int* d_out, si
                o_ctl = take(sizeof(ms::Ctl)), o_mega_v = take(n_mega * 4), o_tasks = take(n_tasks * 8);
   for (auto& q : o_q)
     for (auto& o : q) o = take((size_t)V * 4 + 4);
-  if ((st = grow(w, nz, at))) return st;
-  char* const zero = w.mem.as<char>();
-  char* const rest = zero + w.zero_bytes;
-  if (!w.clean) XBFS_CUDA_TRY(cudaMemsetAsync(zero, 0, w.zero_bytes, s));
+  // a new allocation is not clean, wherever it lies: cudaMalloc may give it the
+  // place of the one just freed
+  if (nz > w.zero.bytes) w.clean = false;
+  if ((st = w.zero.ensure(nz)) || (st = w.rest.ensure(at))) return st;
+  char* const zero = w.zero.as<char>();
+  char* const rest = w.rest.as<char>();
+  if (!w.clean) XBFS_CUDA_TRY(cudaMemsetAsync(zero, 0, w.zero.bytes, s));
   w.clean = false;  // until this traversal has finished
   ms::Params<W> p;
   memset(&p, 0, sizeof(p));
