@@ -459,7 +459,8 @@ __device__ void mlp_stage(const float* __restrict__ w, float* sw) {
 
 // Features (log1p of n_f, m_f, n_u, m_u and the level; the previous
 // strategy; log growth of the frontier; log1p of its mean degree), one per
-// lane, then the three layers with the hidden activations passed by shuffles.
+// lane, then the three layers with the hidden activations passed through shared
+// memory.
 // Called by one full warp.
 // Certified reuse (mlp_reuse_bound, per CTA, in shared memory): the last
 // evaluation's statistics, class and margin (its logit minus the best other,

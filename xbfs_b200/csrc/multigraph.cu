@@ -20,7 +20,8 @@
 //    heavier ones warp-cooperatively; bottom-up gives each lane one unvisited
 //    vertex and stops at the first parent.
 //  * The CTA shape (threads per CTA), the thread/warp degree threshold and the
-//    direction threshold are picked by a small autotuner (xbfs_multi_tune).
+//    direction threshold are picked by a small autotuner (xbfs_multi_tune);
+//    before that, teams and single CTAs have thresholds of their own.
 #include <string.h>
 
 #include <algorithm>
