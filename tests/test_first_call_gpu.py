@@ -46,7 +46,7 @@ def test_first_batch_of_a_handle_and_its_end():
     import torch
     gc.collect()
     batch, many = [], []
-    for i in range(13):
+    for i in range(25):
         g = Graph.rmat(18, 16, 5 + i)
         srcs = pick_sources(g.offsets(), 64, 1)
         lv = torch.empty((64, g.V), dtype=torch.int32, device="cuda:0")

@@ -3243,14 +3243,15 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(const __grid_constant__ Param
       QOut qo;
       for (int b2 = 0; b2 < 3; ++b2) qo.b[b2] = p.q[par ^ 1][b2];
       qo.ctr = F1->bin;
-      // a CTA whose whole share is at most 32 small-bin entries and about
-      // kTinyEdges edges takes the warp-only path (no staging, no block
-      // reductions)
+      // when no CTA's share is over 32 small-bin entries and about kTinyEdges
+      // edges, one warp of each takes it alone (no staging, no block
+      // reductions). All CTAs take the same path: gather_all splits the queue
+      // otherwise, by edges.
       const unsigned long long pk0 = sm.bins[0];
       const unsigned cnt0 = (unsigned)(pk0 & kCountMask);
       const unsigned i0 = (unsigned)((unsigned long long)cnt0 * blockIdx.x / nb);
       const unsigned i1 = (unsigned)((unsigned long long)cnt0 * (blockIdx.x + 1) / nb);
-      const bool tiny = q_valid && (sm.bins[1] & kCountMask) == 0 && (sm.bins[2] & kCountMask) == 0 && i1 - i0 <= 32 &&
+      const bool tiny = q_valid && (sm.bins[1] & kCountMask) == 0 && (sm.bins[2] & kCountMask) == 0 && cnt0 <= 32ull * nb &&
                         (pk0 >> 31) <= (unsigned long long)nb * kTinyEdges;
       if (tiny) {
         if (threadIdx.x < 32 && i1 > i0)
